@@ -6,6 +6,7 @@
 #include "n2p2_b200.h"
 
 #include "kernels.h"
+#include "sf_pair.h"
 #include "potential.h"
 
 #include <algorithm>
@@ -195,6 +196,13 @@ struct n2p2b_context
     std::vector<DevGroup>  tabGroups;    // SF tables (sfp points here)
     std::vector<DevMember> tabMembers;
     DevBuf       tabGroupsDev, tabMembersDev;
+    // Two-pass path (sf_pair.h): values, then forces from dE/dG without
+    // dG/dr.  Off for potentials it does not serve and when a variant of
+    // the general kernels is asked for (N2P2B_SF_VARIANT).
+    PairTables   pt;
+    PairParams   ptDev{};
+    DevBuf       pairTabs;
+    bool         pairEnabled = false;
     NNParams     nnp{};
     int          maxSF = 0;
     int          maxSlots = 0;
@@ -283,6 +291,9 @@ struct n2p2b_context
     // Pipeline state (what the last calls computed).
     bool haveNL = false, haveSF = false, haveSFDeriv = false, haveNN = false;
     bool haveNNDeriv = false, haveE = false, haveF = false;
+    // dG/dr of the current symmetry functions is in dGdr (else it is formed
+    // when something asks for it, and forces come from the two-pass path).
+    bool haveDGdr = false, graphDGdr = false;
 
     // Per-stage device timing (n2p2b_set_profiling).
     bool                     profiling = false;
@@ -367,7 +378,7 @@ struct n2p2b_context
                           &nbrEl, &dx, &dy, &dz, &dd, &entryAtom, &mirror,
                           &pairF, &dGdr, &G, &dEdG, &dGdrSelf, &Ei, &selfF,
                           &F, &energyOut, &status, &tabGroupsDev,
-                          &tabMembersDev})
+                          &tabMembersDev, &pairTabs})
             b->release();
         if (statusHost) cudaFreeHost(statusHost);
         if (energyHost) cudaFreeHost(energyHost);
@@ -699,6 +710,7 @@ struct n2p2b_context
                           cudaMemcpyHostToDevice), "copy SF members");
         sfp.dGroups = tabGroupsDev.as<DevGroup>();
         sfp.dMembers = tabMembersDev.as<DevMember>();
+        buildPair();
         sfScale.ensure(sizeof(SFScale) * scale.size());
         ck(cudaMemcpy(sfScale.p, scale.data(), sizeof(SFScale) * scale.size(),
                       cudaMemcpyHostToDevice), "copy SF scaling");
@@ -730,6 +742,46 @@ struct n2p2b_context
         invalidate();
     }
 
+    // Tables of the two-pass path, uploaded as one blob.
+    void buildPair()
+    {
+        buildPairTables(sfp, pt);
+        pairEnabled = pt.ok && !std::getenv("N2P2B_SF_VARIANT");
+        if (!pairEnabled) return;
+        std::vector<unsigned char> blob;
+        auto add = [&](auto const& v) {
+            std::size_t const at = blob.size();
+            auto const* p = reinterpret_cast<unsigned char const*>(v.data());
+            blob.insert(blob.end(), p, p + sizeof(v[0]) * v.size());
+            blob.resize((blob.size() + 15) / 16 * 16);
+            return at;
+        };
+        std::size_t const u = add(pt.units), r = add(pt.runs),
+                          h = add(pt.shapes), q = add(pt.radials),
+                          c = add(pt.cells), f = add(pt.fcs), w = add(pt.rads);
+        pt.p.units = pt.units.data();
+        pairTabs.ensure(std::max<std::size_t>(blob.size(), 16));
+        if (!blob.empty())
+            ck(cudaMemcpy(pairTabs.p, blob.data(), blob.size(),
+                          cudaMemcpyHostToDevice), "copy pair tables");
+        unsigned char const* d = pairTabs.as<unsigned char>();
+        ptDev = pt.p;
+        ptDev.units = reinterpret_cast<PairUnit const*>(d + u);
+        ptDev.runs = reinterpret_cast<PairRun const*>(d + r);
+        ptDev.shapesTab = reinterpret_cast<PairShape const*>(d + h);
+        ptDev.radials = reinterpret_cast<PairRadial const*>(d + q);
+        ptDev.cells = reinterpret_cast<PairCell const*>(d + c);
+        ptDev.fcs = reinterpret_cast<PairFc const*>(d + f);
+        ptDev.rads = reinterpret_cast<PairRad const*>(d + w);
+    }
+
+    // The two-pass path serves the potential and the current staging
+    // capacity fits its shared memory.
+    bool pairUsable() const
+    {
+        return pairEnabled && pairFits(pt.p, sfCap, precision, maxSF);
+    }
+
     void requireReady() const
     {
         if (!generic || !scaled || !weighted || !tablesReady)
@@ -751,7 +803,7 @@ struct n2p2b_context
     void invalidate()
     {
         haveNL = haveSF = haveSFDeriv = haveNN = haveNNDeriv = false;
-        haveE = haveF = false;
+        haveE = haveF = haveDGdr = false;
     }
 
     // ---- structure -------------------------------------------------------
@@ -1071,7 +1123,11 @@ struct n2p2b_context
         entryAtom.ensure(sizeof(int) * c);
         mirror.ensure(sizeof(int) * c);
         pairF.ensure(sizeof(double) * 3 * c);
-        dGdr.ensure(realBytes() * 3 * (std::size_t)c
+    }
+
+    void ensureDGdr()
+    {
+        dGdr.ensure(realBytes() * 3 * (std::size_t)std::max(capacity, 1L)
                     * std::max(maxSlots, 1));
     }
 
@@ -1215,8 +1271,73 @@ struct n2p2b_context
         launchNeighborList(L, stream);
     }
 
-    void enqueueSF(bool deriv)
+    PairLaunch pairLaunch()
     {
+        if (smCount == 0)
+            ck(cudaDeviceGetAttribute(&smCount, cudaDevAttrMultiProcessorCount,
+                                      device), "device attribute");
+        PairLaunch L;
+        L.n = (int)n;
+        L.cap = sfCap;
+        L.sms = smCount;
+        L.precision = precision;
+        L.maxSF = maxSF;
+        L.elem = elem.as<int>();
+        L.nbrOff = nbrOff.as<int>();
+        L.nbrCountElem = nbrCountElem.as<int>();
+        L.dx = dx.as<double>();
+        L.dy = dy.as<double>();
+        L.dz = dz.as<double>();
+        L.dd = dd.as<double>();
+        L.scale = sfScale.as<SFScale>();
+        L.G = G.p;
+        L.dEdG = dEdG.p;
+        L.pairF = pairF.as<double>();
+        L.selfF = selfF.as<double>();
+        L.status = status.as<int>();
+        return L;
+    }
+
+    // Symmetry functions; with `store` also dG/dr in memory.  Without it the
+    // two-pass path computes the values (where it serves) and the forces are
+    // left to its second pass.
+    void enqueueSF(bool deriv, bool store)
+    {
+        if (!store && pairUsable())
+        {
+            launchPair(0, sfp, pt.p, ptDev, pairLaunch(), stream);
+            haveDGdr = false;
+            return;
+        }
+        enqueueStoredSF(deriv, G.p);
+        haveDGdr = deriv;
+    }
+
+    // dG/dr of the current symmetry functions, if the evaluation left it out
+    // (the values that the networks saw stay as they are).
+    void requireDGdr()
+    {
+        if (haveDGdr) return;
+        DevBuf scratch;
+        try
+        {
+            scratch.ensure(realBytes() * n * maxSF);
+            enqueueStoredSF(true, scratch.p);
+            checkLaunch("symmetry-function derivatives");
+            ck(cudaStreamSynchronize(stream), "synchronize");
+        }
+        catch (...)
+        {
+            scratch.release();
+            throw;
+        }
+        scratch.release();
+        haveDGdr = true;
+    }
+
+    void enqueueStoredSF(bool deriv, void* outG)
+    {
+        if (deriv) ensureDGdr();
         if (sfVariant < 0)
         {
             sfVariant = sfDefaultVariant(sfp, precision);
@@ -1252,7 +1373,7 @@ struct n2p2b_context
         L.dd = dd.as<double>();
         L.scale = sfScale.as<SFScale>();
         L.precision = precision;
-        L.G = G.p;
+        L.G = outG;
         L.dGdr = dGdr.p;
         L.status = status.as<int>();
         launchSymmetryFunctions(sfp, L, stream);
@@ -1626,6 +1747,7 @@ struct n2p2b_context
         if (batchSize <= 0 || !labelE || !labelF || !batch)
             throw std::invalid_argument("ERROR: Bad training batch.\n");
         activate();
+        requireDGdr();
         enqueueStudentNN(true);
         enqueueForces();
         stu.rE.ensure(sizeof(float) * n);
@@ -1902,6 +2024,8 @@ struct n2p2b_context
     {
         ForceLaunch L = forceLaunch();
         L.gather = externalNL ? 0 : 1;
+        L.terms = haveDGdr ? 1 : 0;
+        if (!haveDGdr) launchPair(1, sfp, pt.p, ptDev, pairLaunch(), stream);
         launchForces(L, stream);
         if (!externalNL) return;
         TargetForceLaunch T;
@@ -2114,7 +2238,10 @@ struct n2p2b_context
             if (st & 1) { enqueueNL(); mark(1); }
             if (st & 2)
             {
-                enqueueSF(sfDeriv);
+                // An evaluation with forces (or without derivatives) needs
+                // no dG/dr in memory; the symmetry-function step alone
+                // leaves it there.
+                enqueueSF(sfDeriv, sfDeriv && !(stages & 16));
                 if (ewCheck) enqueueEW();
                 mark(2);
             }
@@ -2177,7 +2304,7 @@ struct n2p2b_context
         beginProfile();
         enqueueNL();
         mark(1);
-        enqueueSF(forces);
+        enqueueSF(forces, false);
         if (ewCheck) enqueueEW();
         mark(2);
         enqueueNN(forces);
@@ -2255,6 +2382,7 @@ struct n2p2b_context
         ck(e, "instantiate graph");
         graphValid = true;
         graphForces = forces;
+        graphDGdr = haveDGdr;
     }
 
     void launchGraph()
@@ -2266,6 +2394,7 @@ struct n2p2b_context
         ck(cudaGraphLaunch(graphExec, stream), "launch graph");
         invalidate();
         haveSFDeriv = haveNNDeriv = haveF = graphForces;
+        haveDGdr = graphDGdr;
     }
 
     // ---- autotuner ----------------------------------------------------------
@@ -2346,10 +2475,15 @@ struct n2p2b_context
         double const t0 = timeIt();
         TuneChoice best{sfVariant, sfSortCats, nlWarpsPerBlock, t0};
         std::string rep;
+        // The two-pass path has no variants: only the neighbor list's
+        // launch is left to choose.
+        bool const pair = pairUsable();
         for (int v = 0; v < kSFVariants; ++v)
             for (int so : {1, 3, 5, 7})
                 for (int w : nls)
                 {
+                    if (pair && (v != start.variant || so != start.sortCats))
+                        continue;
                     // The staged kernel ignores the item order.
                     if (v >= 6 && so != 5) continue;
                     sfVariant = v;
@@ -3190,6 +3324,7 @@ int n2p2b_get_dGdr(n2p2b_context* ctx, double* self, int sfStride,
         if (sfStride < ctx->maxSF || slotStride < ctx->maxSlots)
             throw std::invalid_argument("ERROR: stride");
         ctx->activate();
+        ctx->requireDGdr();
         long const n = ctx->n;
         int const S = ctx->maxSlots;
         if (self)

@@ -399,6 +399,7 @@ struct ForceLaunch
     double*        F = nullptr;       // [n][3] output (physical units)
     double         forceScale = 1.0;  // divide by (convEnergy / convLength)
     int            gather = 1;        // 0: pair and self terms only
+    int            terms = 1;         // 0: pair and self terms are in place
     int const*     status = nullptr;
 };
 

@@ -570,10 +570,10 @@ void launchForces(ForceLaunch const& L, cudaStream_t s)
     std::size_t const shm = sizeof(double) * warps
                           * (std::size_t)(L.maxSF + L.numElements * L.maxSlots);
     int const grid = (L.n + warps - 1) / warps;
-    noteLaunches(L.gather ? 2 : 1);
-    if (L.precision != PREC_FP64)
+    noteLaunches((L.terms ? 1 : 0) + (L.gather ? 1 : 0));
+    if (L.terms && L.precision != PREC_FP64)
         pairForceKernel<float><<<grid > 0 ? grid : 1, 32 * warps, shm, s>>>(L);
-    else
+    else if (L.terms)
         pairForceKernel<double><<<grid > 0 ? grid : 1, 32 * warps, shm, s>>>(L);
     if (!L.gather) return;
     int const tb = 256;    // 8 atoms (warps) per block

@@ -1,0 +1,9 @@
+// Two-pass symmetry-function kernels, FP32 (mixed forms).
+#include "sf_pair_launch.cuh"
+
+namespace n2p2b
+{
+
+N2P2B_PAIR_LAUNCH(tanhu4f, float, 2, 5, (sfp2::kHasPow2), 5, 6)
+
+} // namespace n2p2b
