@@ -21,6 +21,8 @@
 #include <sstream>
 #include <stdexcept>
 #include <string>
+#include <system_error>
+#include <thread>
 #include <map>
 #include <vector>
 
@@ -80,6 +82,105 @@ struct DevBuf
         bytes = 0;
     }
     template <typename T> T* as() const { return static_cast<T*>(p); }
+};
+
+// Copies large pageable host arrays to the device through small pinned
+// buffers, a few host threads filling them while the copy engine drains them
+// (one thread alone is bound by its memcpy).  Pinned memory: kThreads x
+// kBufs x kChunk = 8 MB per context, allocated at the first use and released
+// with the context; only that context's calls use it.
+struct Uploader
+{
+    static constexpr int kThreads = 4, kBufs = 2;
+    static constexpr std::size_t kChunk = std::size_t(1) << 20;
+
+    struct Job
+    {
+        void*       dst;
+        void const* src;
+        std::size_t bytes;
+    };
+
+    unsigned char* pinned = nullptr;
+    cudaEvent_t    done[kThreads][kBufs] = {};
+
+    void copy(int device, cudaStream_t stream, std::vector<Job> const& jobs)
+    {
+        std::size_t total = 0;
+        for (Job const& j : jobs) total += j.bytes;
+        if (total < 2 * kChunk)
+        {
+            for (Job const& j : jobs)
+                if (j.bytes)
+                    ck(cudaMemcpyAsync(j.dst, j.src, j.bytes,
+                                       cudaMemcpyHostToDevice, stream),
+                       "upload");
+            return;
+        }
+        if (!pinned)
+        {
+            for (auto& t : done)
+                for (cudaEvent_t& e : t)
+                    if (!e)
+                        ck(cudaEventCreateWithFlags(
+                               &e, cudaEventDisableTiming), "event");
+            ck(cudaMallocHost((void**)&pinned, kThreads * kBufs * kChunk),
+               "cudaMallocHost");
+        }
+        // Chunks of all jobs, dealt to the threads in turn.
+        std::vector<Job> chunks;
+        for (Job const& j : jobs)
+            for (std::size_t o = 0; o < j.bytes; o += kChunk)
+                chunks.push_back(Job{
+                    static_cast<unsigned char*>(j.dst) + o,
+                    static_cast<unsigned char const*>(j.src) + o,
+                    std::min(kChunk, j.bytes - o)});
+        cudaError_t err[kThreads] = {};
+        auto work = [&](int t) {
+            cudaError_t e = cudaSetDevice(device);
+            int slot = 0;
+            for (std::size_t k = t; k < chunks.size() && e == cudaSuccess;
+                 k += kThreads, slot ^= 1)
+            {
+                unsigned char* buf = pinned + (t * kBufs + slot) * kChunk;
+                // The copy that last read this buffer (none: returns).
+                e = cudaEventSynchronize(done[t][slot]);
+                if (e != cudaSuccess) break;
+                std::memcpy(buf, chunks[k].src, chunks[k].bytes);
+                e = cudaMemcpyAsync(chunks[k].dst, buf, chunks[k].bytes,
+                                    cudaMemcpyHostToDevice, stream);
+                if (e == cudaSuccess)
+                    e = cudaEventRecord(done[t][slot], stream);
+            }
+            err[t] = e;
+        };
+        std::vector<std::thread> threads;
+        try
+        {
+            for (int t = 1; t < kThreads; ++t) threads.emplace_back(work, t);
+        }
+        catch (std::system_error const&)
+        {
+            // No more threads to be had: this one does their shares too.
+        }
+        int const started = 1 + (int)threads.size();
+        work(0);
+        for (auto& t : threads) t.join();
+        for (int t = started; t < kThreads; ++t) work(t);
+        for (cudaError_t e : err) ck(e, "upload");
+    }
+
+    void release()
+    {
+        for (auto& t : done)
+            for (cudaEvent_t& e : t)
+            {
+                if (e) cudaEventDestroy(e);
+                e = nullptr;
+            }
+        if (pinned) cudaFreeHost(pinned);
+        pinned = nullptr;
+    }
 };
 
 // --- reference geometry (libnnp/Vec3D.h, Structure.cpp) --------------------
@@ -228,7 +329,8 @@ struct n2p2b_context
     // Externally supplied neighbor list (n2p2b_set_neighbor_list).
     bool         externalNL = false;
     long         numTargets = 0;
-    DevBuf       revOff, revEntry, Ftarget;
+    DevBuf       revOff, revEntry, Ftarget, engRaw, engScratch;
+    Uploader     engUp;
 
     // Batch of independent structures (numStructs > 0).
     long         numStructs = 0;
@@ -363,7 +465,7 @@ struct n2p2b_context
             for (auto& e : se.ev) cudaEventDestroy(e);
         if (graphExec) cudaGraphExecDestroy(graphExec);
         for (DevBuf* b : {&structOf, &structAtoms, &bsDev, &structEnergy,
-                          &revOff, &revEntry, &Ftarget})
+                          &revOff, &revEntry, &Ftarget, &engRaw, &engScratch})
             b->release();
         for (DevBuf* b : {&stu.w, &stu.m, &stu.v, &stu.grad, &stu.gpart,
                           &stu.rE,
@@ -380,6 +482,7 @@ struct n2p2b_context
                           &F, &energyOut, &status, &tabGroupsDev,
                           &tabMembersDev, &pairTabs})
             b->release();
+        engUp.release();
         if (statusHost) cudaFreeHost(statusHost);
         if (energyHost) cudaFreeHost(energyHost);
         if (ownStream && stream) cudaStreamDestroy(stream);
@@ -2118,45 +2221,13 @@ struct n2p2b_context
         }
         es.start[ne] = (int)byElem.size();
         for (int e = ne + 1; e <= kMaxElem; ++e) es.start[e] = es.start[ne];
-        double const L = pot.normalize ? pot.convLength : 1.0;
-        std::vector<int> off(n + 1, 0), cntE((std::size_t)n * ne, 0);
-        std::vector<int> idx(E), rev((std::size_t)targets + 1, 0);
-        std::vector<int8_t> el(E);
-        std::vector<double> x(E), y(E), z(E), d(E);
+        std::vector<int> off(n + 1, 0);
         int maxCnt = 0;
-        long src = 0;
         for (long i = 0; i < n; ++i)
         {
             off[i + 1] = off[i] + (int)counts[i];
             maxCnt = std::max(maxCnt, (int)counts[i]);
-            long dst = off[i];
-            for (int e = 0; e < ne; ++e)
-                for (long k = src; k < src + counts[i]; ++k)
-                {
-                    if (nelems[k] < 0 || nelems[k] >= ne || index[k] < 0
-                        || index[k] >= targets)
-                        throw std::invalid_argument("ERROR: Bad neighbor "
-                                                    "entry.\n");
-                    if (nelems[k] != e) continue;
-                    double const a = drIn[3 * k], b = drIn[3 * k + 1],
-                                 c = drIn[3 * k + 2];
-                    idx[dst] = (int)index[k];
-                    el[dst] = (int8_t)e;
-                    // InterfaceLammps::addNeighbor: n.d = sqrt(d2), scaled
-                    // like the components.
-                    d[dst] = std::sqrt(a * a + b * b + c * c) * L;
-                    x[dst] = a * L;
-                    y[dst] = b * L;
-                    z[dst] = c * L;
-                    ++cntE[(std::size_t)i * ne + e];
-                    ++rev[idx[dst] + 1];
-                    ++dst;
-                }
-            src += counts[i];
         }
-        for (long m = 0; m < targets; ++m) rev[m + 1] += rev[m];
-        std::vector<int> fill(rev.begin(), rev.end() - 1), revE(E);
-        for (long e = 0; e < E; ++e) revE[fill[idx[e]]++] = (int)e;
         ensureStructureBuffers();
         capacity = std::max(capacity, std::max(E, 1L));
         ensureEntryBuffers();
@@ -2165,6 +2236,37 @@ struct n2p2b_context
         revOff.ensure(sizeof(int) * (targets + 1));
         revEntry.ensure(sizeof(int) * std::max(E, 1L));
         Ftarget.ensure(sizeof(double) * 3 * targets);
+        engRaw.ensure(36 * (std::size_t)std::max(E, 1L));
+        engScratch.ensure(sizeof(int) * (std::size_t)(targets + 1 + E));
+        invalidate();
+        EngineListLaunch G;
+        G.n = n;
+        G.entries = E;
+        G.numElements = ne;
+        G.numTargets = targets;
+        G.scale = pot.normalize ? pot.convLength : 1.0;
+        G.off = nbrOff.as<int>();
+        // Raw entries: displacements, indices, elements.
+        unsigned char* const raw = engRaw.as<unsigned char>();
+        G.rawDr = reinterpret_cast<double const*>(raw);
+        G.rawIndex = reinterpret_cast<int64_t const*>(raw + 24 * E);
+        G.rawElem = reinterpret_cast<int const*>(raw + 32 * E);
+        G.nbrCountElem = nbrCountElem.as<int>();
+        G.nbrIdx = nbrIdx.as<int>();
+        G.nbrEl = nbrEl.as<int8_t>();
+        G.dx = dx.as<double>();
+        G.dy = dy.as<double>();
+        G.dz = dz.as<double>();
+        G.dd = dd.as<double>();
+        G.bad = engScratch.as<int>();
+        G.revCount = engScratch.as<int>() + 1;
+        G.revTmp = engScratch.as<int>() + 1 + targets;
+        G.revOff = revOff.as<int>();
+        G.revEntry = revEntry.as<int>();
+        engUp.copy(device, stream,
+                   {{raw, drIn, 24 * (std::size_t)E},
+                    {raw + 24 * E, index, 8 * (std::size_t)E},
+                    {raw + 32 * E, nelems, 4 * (std::size_t)E}});
         auto up = [&](DevBuf& b, void const* h, std::size_t bytes) {
             if (bytes)
                 ck(cudaMemcpyAsync(b.p, h, bytes, cudaMemcpyHostToDevice,
@@ -2173,16 +2275,14 @@ struct n2p2b_context
         up(elem, elemHost.data(), sizeof(int) * n);
         up(atomsByElem, byElem.data(), sizeof(int) * n);
         up(nbrOff, off.data(), sizeof(int) * (n + 1));
-        up(nbrCountElem, cntE.data(), sizeof(int) * cntE.size());
-        up(nbrIdx, idx.data(), sizeof(int) * E);
-        up(nbrEl, el.data(), E);
-        up(dx, x.data(), sizeof(double) * E);
-        up(dy, y.data(), sizeof(double) * E);
-        up(dz, z.data(), sizeof(double) * E);
-        up(dd, d.data(), sizeof(double) * E);
-        up(revOff, rev.data(), sizeof(int) * (targets + 1));
-        up(revEntry, revE.data(), sizeof(int) * E);
+        launchEngineList(G, stream);
+        checkLaunch("neighbor list kernels");
+        int bad = 0;
+        ck(cudaMemcpyAsync(&bad, G.bad, sizeof(int), cudaMemcpyDeviceToHost,
+                           stream), "read neighbor list check");
         ck(cudaStreamSynchronize(stream), "neighbor list upload");
+        if (bad)
+            throw std::invalid_argument("ERROR: Bad neighbor entry.\n");
         invalidate();
         haveNL = true;
         lastMaxNbr = maxCnt;

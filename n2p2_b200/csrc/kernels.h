@@ -55,6 +55,37 @@ struct NLLaunch
     int*                status = nullptr;
 };
 
+// An MD engine's neighbor list (kernels_engine.cu): raw entries in the
+// engine's order and what they become.
+struct EngineListLaunch
+{
+    long           n = 0;              // local atoms
+    long           entries = 0;
+    int            numElements = 0;
+    long           numTargets = 0;
+    double         scale = 1.0;        // physical -> computing length unit
+    int const*     off = nullptr;      // [n + 1]
+    int64_t const* rawIndex = nullptr; // [entries]
+    int const*     rawElem = nullptr;
+    double const*  rawDr = nullptr;    // [entries][3]
+    int*           nbrCountElem = nullptr;
+    int*           nbrIdx = nullptr;
+    int8_t*        nbrEl = nullptr;
+    double*        dx = nullptr;
+    double*        dy = nullptr;
+    double*        dz = nullptr;
+    double*        dd = nullptr;
+    int*           revCount = nullptr; // [numTargets] scratch
+    int*           revOff = nullptr;   // [numTargets + 1]
+    int*           revTmp = nullptr;   // [entries] scratch
+    int*           revEntry = nullptr; // [entries]
+    int*           bad = nullptr;      // set if an entry is out of range
+};
+
+void launchEngineList(EngineListLaunch const& L, cudaStream_t s);
+// off[0 .. n] = exclusive prefix sums of cnt[0 .. n).
+void launchOffsetScan(long n, int const* cnt, int* off, cudaStream_t s);
+
 // Running count of kernel launches issued by this library (diagnostics).
 void noteLaunches(int k);
 

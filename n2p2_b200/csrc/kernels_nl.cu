@@ -380,52 +380,75 @@ __global__ void nlBruteKernel(int n, NLParams p, int numElements,
 // Exclusive scan of per-atom counts into offsets (n + 1 entries), total and
 // maximum into the status words; flags overflow against `capacity`.
 // Single block; each thread scans a contiguous chunk.
-__global__ void nlScanKernel(int n, int const* __restrict__ cnt,
-                             int* __restrict__ off, long capacity,
-                             int* __restrict__ status)
+__global__ void __launch_bounds__(1024)
+nlScanKernel(int n, int const* __restrict__ cnt, int* __restrict__ off,
+             long capacity, int* __restrict__ status)
 {
-    __shared__ long sPart[1024];
-    __shared__ int sMax[1024];
-    int const t = threadIdx.x;
-    int const T = blockDim.x;
-    int const chunk = (n + T - 1) / T;
-    int const b = min(n, t * chunk);
-    int const e = min(n, b + chunk);
-    long s = 0;
+    __shared__ int sWarp[32];
+    __shared__ int sMax[32];
+    constexpr int kPer = 8;               // consecutive counts per thread
+    int const t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    long base = 0;
     int mx = 0;
-    for (int i = b; i < e; ++i)
+    for (int tile = 0; tile < n; tile += 1024 * kPer)
     {
-        s += cnt[i];
-        mx = max(mx, cnt[i]);
-    }
-    sPart[t] = s;
-    sMax[t] = mx;
-    __syncthreads();
-    if (t == 0)
-    {
-        long run = 0;
-        int m = 0;
-        for (int k = 0; k < T; ++k)
+        int const b = tile + t * kPer;
+        int v[kPer], s = 0;
+#pragma unroll
+        for (int k = 0; k < kPer; ++k)
         {
-            long const v = sPart[k];
-            sPart[k] = run;
-            run += v;
-            m = max(m, sMax[k]);
+            v[k] = b + k < n ? cnt[b + k] : 0;
+            mx = max(mx, v[k]);
+            s += v[k];
         }
-        off[n] = (int)min(run, (long)0x7fffffff);
-        status[ST_TOTAL_NBR] = (int)min(run, (long)0x7fffffff);
-        status[ST_MAX_NBR] = m;
-        if (run > capacity)
+        int incl = s;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1)
         {
-            status[ST_FLAGS] |= FLAG_NBR_OVERFLOW | FLAG_ABORT;
+            int const u = __shfl_up_sync(0xffffffffu, incl, d);
+            if (lane >= d) incl += u;
         }
+        if (lane == 31) sWarp[warp] = incl;
+        __syncthreads();
+        if (warp == 0)
+        {
+            int w = sWarp[lane];
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1)
+            {
+                int const u = __shfl_up_sync(0xffffffffu, w, d);
+                if (lane >= d) w += u;
+            }
+            sWarp[lane] = w;
+        }
+        __syncthreads();
+        long run = base + (warp > 0 ? sWarp[warp - 1] : 0) + incl - s;
+        base += sWarp[31];
+#pragma unroll
+        for (int k = 0; k < kPer; ++k)
+        {
+            if (b + k < n) off[b + k] = (int)run;
+            run += v[k];
+        }
+        __syncthreads();
     }
+    mx = __reduce_max_sync(0xffffffffu, mx);
+    if (lane == 0) sMax[warp] = mx;
     __syncthreads();
-    long run = sPart[t];
-    for (int i = b; i < e; ++i)
+    if (warp == 0)
     {
-        off[i] = (int)run;
-        run += cnt[i];
+        int const m = __reduce_max_sync(0xffffffffu, sMax[lane]);
+        if (lane == 0)
+        {
+            off[n] = (int)min(base, (long)0x7fffffff);
+            if (status)
+            {
+                status[ST_TOTAL_NBR] = (int)min(base, (long)0x7fffffff);
+                status[ST_MAX_NBR] = m;
+                if (base > capacity)
+                    status[ST_FLAGS] |= FLAG_NBR_OVERFLOW | FLAG_ABORT;
+            }
+        }
     }
 }
 
@@ -541,6 +564,12 @@ __global__ void nlEntryAtomKernel(int n, int const* __restrict__ nbrOff,
 // ---------------------------------------------------------------------------
 // Host-side launchers
 // ---------------------------------------------------------------------------
+
+void launchOffsetScan(long n, int const* cnt, int* off, cudaStream_t s)
+{
+    nlScanKernel<<<1, 1024, 0, s>>>((int)n, cnt, off, 0x7fffffffffffffffL,
+                                    nullptr);
+}
 
 void launchNeighborList(NLLaunch const& L, cudaStream_t s)
 {
