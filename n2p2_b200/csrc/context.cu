@@ -257,10 +257,12 @@ void pbcCopies(double const box[3][3], double rc, int pbc[3], double proj[3])
     }
 }
 
-__global__ void statusResetKernel(int* status)
+__global__ void statusResetKernel(int* status, int* cellStatus)
 {
-    if (threadIdx.x < ST_NUM) status[threadIdx.x] = 0;
-    if (threadIdx.x == ST_BAD_ATOM) status[threadIdx.x] = -1;
+    if (threadIdx.x >= ST_NUM) return;
+    int const v = threadIdx.x == ST_BAD_ATOM ? -1 : 0;
+    status[threadIdx.x] = v;
+    cellStatus[threadIdx.x] = v;
 }
 
 std::atomic<unsigned long long> g_launches{0};
@@ -1296,15 +1298,20 @@ struct n2p2b_context
 
     void enqueueReset()
     {
-        noteLaunches(2);
-        statusResetKernel<<<1, 32, 0, stream>>>(status.as<int>());
-        statusResetKernel<<<1, 32, 0, stream>>>(cellStatus.as<int>());
+        noteLaunches(1);
+        statusResetKernel<<<1, 32, 0, stream>>>(status.as<int>(),
+                                                cellStatus.as<int>());
     }
 
     void enqueueNL()
     {
         if (externalNL) return;      // the caller's list is already in place
-        if (numStructs > 0)
+        // Small single structures run as a batch of one: every pair of atoms
+        // is a candidate, but there are no cells to build and the entries
+        // come in key order (nothing to sort).  192 atoms 0.206 -> 0.044 ms,
+        // 1,080 atoms 0.148 -> 0.110 ms, 1,728 atoms 0.111 -> 0.130 ms.
+        bool const small = numStructs == 0 && n <= 1536 && nlp.nimg <= 128;
+        if (numStructs > 0 || small)
         {
             NLBatchLaunch B;
             B.n = (int)n;
@@ -1333,6 +1340,19 @@ struct n2p2b_context
             B.entryAtom = entryAtom.as<int>();
             B.mirror = mirror.as<int>();
             B.status = status.as<int>();
+            if (small)
+            {
+                B.NIMG = nlp.nimg;
+                B.warpsPerBlock = n < 1024 ? 1 : 4;
+                B.bs = nullptr;
+                B.structOf = nullptr;
+                B.one.p = nlp;
+                B.one.pb = pb;
+                B.one.doRemap = remap ? 1 : 0;
+                for (int e = 0; e <= kMaxElem; ++e)
+                    B.one.es[e] = es.start[e];
+                B.structAtoms = atomsByElem.as<int>();
+            }
             launchNeighborListBatch(B, stream);
             return;
         }
@@ -2258,9 +2278,10 @@ struct n2p2b_context
         G.dy = dy.as<double>();
         G.dz = dz.as<double>();
         G.dd = dd.as<double>();
-        G.bad = engScratch.as<int>();
-        G.revCount = engScratch.as<int>() + 1;
-        G.revTmp = engScratch.as<int>() + 1 + targets;
+        // The counts first: the scan reads them as 16-byte vectors.
+        G.revCount = engScratch.as<int>();
+        G.revTmp = engScratch.as<int>() + targets;
+        G.bad = engScratch.as<int>() + targets + E;
         G.revOff = revOff.as<int>();
         G.revEntry = revEntry.as<int>();
         engUp.copy(device, stream,

@@ -83,7 +83,7 @@ struct EngineListLaunch
 };
 
 void launchEngineList(EngineListLaunch const& L, cudaStream_t s);
-// off[0 .. n] = exclusive prefix sums of cnt[0 .. n).
+// off[0 .. n] = exclusive prefix sums of cnt[0 .. n); both 16-byte aligned.
 void launchOffsetScan(long n, int const* cnt, int* off, cudaStream_t s);
 
 // Running count of kernel launches issued by this library (diagnostics).
@@ -112,7 +112,9 @@ struct NLBatchLaunch
     int                 normalize = 0;
     double              convLength = 1.0;
     BatchStruct const*  bs = nullptr;
-    int const*          structOf = nullptr;  // [n] structure of each atom
+    int const*          structOf = nullptr;  // [n] structure of each atom;
+                                             // null: all of `one`
+    BatchStruct         one{};               // a single structure
     int const*          structAtoms = nullptr;
     double const*       posIn = nullptr;
     double*             pos = nullptr;

@@ -379,7 +379,8 @@ __global__ void nlBruteKernel(int n, NLParams p, int numElements,
 
 // Exclusive scan of per-atom counts into offsets (n + 1 entries), total and
 // maximum into the status words; flags overflow against `capacity`.
-// Single block; each thread scans a contiguous chunk.
+// Single block: tiles of 8,192 counts, eight per thread, warp scans.  cnt and
+// off are 16-byte aligned (cudaMalloc'ed arrays).
 __global__ void __launch_bounds__(1024)
 nlScanKernel(int n, int const* __restrict__ cnt, int* __restrict__ off,
              long capacity, int* __restrict__ status)
@@ -390,17 +391,35 @@ nlScanKernel(int n, int const* __restrict__ cnt, int* __restrict__ off,
     int const t = threadIdx.x, lane = t & 31, warp = t >> 5;
     long base = 0;
     int mx = 0;
+    // A tile's counts are fetched while the tile before it is scanned.
+    int v[kPer], nx[kPer];
+    auto fetch = [&](int (&x)[kPer], int b) {
+        if (b + kPer <= n)
+        {
+            int4 const p = *reinterpret_cast<int4 const*>(cnt + b);
+            int4 const q = *reinterpret_cast<int4 const*>(cnt + b + 4);
+            x[0] = p.x; x[1] = p.y; x[2] = p.z; x[3] = p.w;
+            x[4] = q.x; x[5] = q.y; x[6] = q.z; x[7] = q.w;
+        }
+        else
+        {
+#pragma unroll
+            for (int k = 0; k < kPer; ++k) x[k] = b + k < n ? cnt[b + k] : 0;
+        }
+    };
+    fetch(nx, t * kPer);
     for (int tile = 0; tile < n; tile += 1024 * kPer)
     {
         int const b = tile + t * kPer;
-        int v[kPer], s = 0;
+        int s = 0;
 #pragma unroll
         for (int k = 0; k < kPer; ++k)
         {
-            v[k] = b + k < n ? cnt[b + k] : 0;
+            v[k] = nx[k];
             mx = max(mx, v[k]);
             s += v[k];
         }
+        if (tile < n - 1024 * kPer) fetch(nx, b + 1024 * kPer);
         int incl = s;
 #pragma unroll
         for (int d = 1; d < 32; d <<= 1)
@@ -424,11 +443,25 @@ nlScanKernel(int n, int const* __restrict__ cnt, int* __restrict__ off,
         __syncthreads();
         long run = base + (warp > 0 ? sWarp[warp - 1] : 0) + incl - s;
         base += sWarp[31];
+        int o[kPer];
 #pragma unroll
         for (int k = 0; k < kPer; ++k)
         {
-            if (b + k < n) off[b + k] = (int)run;
+            o[k] = (int)run;
             run += v[k];
+        }
+        if (b + kPer <= n)
+        {
+            *reinterpret_cast<int4*>(off + b) = make_int4(o[0], o[1], o[2],
+                                                          o[3]);
+            *reinterpret_cast<int4*>(off + b + 4) = make_int4(o[4], o[5],
+                                                              o[6], o[7]);
+        }
+        else
+        {
+#pragma unroll
+            for (int k = 0; k < kPer; ++k)
+                if (b + k < n) off[b + k] = o[k];
         }
         __syncthreads();
     }
@@ -639,12 +672,13 @@ void launchNeighborList(NLLaunch const& L, cudaStream_t s)
 __global__ void nlbPrepareKernel(int n, double const* __restrict__ posIn,
                                  int const* __restrict__ structOf,
                                  BatchStruct const* __restrict__ bs,
+                                 __grid_constant__ BatchStruct const one,
                                  int normalize, double convLength,
                                  double* __restrict__ pos)
 {
     int const i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    BatchStruct const& S = bs[structOf[i]];
+    BatchStruct const& S = structOf ? bs[structOf[i]] : one;
     double r[3] = {posIn[3 * i + 0], posIn[3 * i + 1], posIn[3 * i + 2]};
     if (S.doRemap) remapAtom(r, S.pb.box, S.pb.invbox);
     if (normalize)
@@ -800,52 +834,79 @@ __global__ void nlbMirrorKernel(int n, int NIMG,
     }
 }
 
-// Batch neighbor list, faster form of nlbBruteKernel for structures with at
-// most 128 images (|bc| <= 2 per box vector): warp per atom i, lanes over
-// the candidates j of one element (positions loaded once), each lane walks
-// the structure's images in key order with an incremental (b0, b1, b2)
-// counter.  An FP32 distance test only filters: its threshold rc^2 + m
-// covers the FP32 rounding of the displacement and image-shift sums (m from
-// a bound on their magnitudes, at least 1e-4 rc^2), and every candidate it
-// keeps gets the exact FP64 test of nlTest, so the neighbor sets are those
-// of the brute path.  Hits are kept
-// as per-lane image bit masks and written in key order (lane = j
-// ascending, bits = image ascending) through a warp prefix sum.
+// Neighbor list of batches and of small single structures with at most 128
+// images: warp per atom i, lanes over the candidates j of one element
+// (positions loaded once).  A lane walks only the images that can be in
+// reach: with s_k the fractional coordinate of r_i - r_j along box vector k
+// and w_k the distance between the cell's faces, an image b is at least
+// |s_k + b_k| w_k away, so b_k runs from ceil(-rc / w_k - s_k) to
+// floor(rc / w_k - s_k) inside [-pbc_k, pbc_k] (in FP32, widened by far more
+// than its error): 1 to 8 images instead of 27.  An FP32 distance decides
+// outside rc^2 -+ m, where m covers the FP32 rounding of the displacement and
+// image-shift sums (m from a bound on their magnitudes, at least 1e-4 rc^2);
+// between them the exact FP64 test of nlTest does, so the neighbor sets are
+// those of the brute path.  Hits are kept
+// as per-lane image bit masks and placed in key order (lane = j ascending,
+// bits = image ascending) through a warp prefix sum; MODE 0 counts, MODE 1
+// writes the entries.  384 water boxes (101,160 atoms), both passes and
+// the entries: 3.7 ms with all 27 images, 1.1 ms so.
+struct LaneOut
+{
+    unsigned long long* key;
+    int*                nbrIdx;
+    int8_t*             nbrEl;
+    double*             dx;
+    double*             dy;
+    double*             dz;
+    double*             dd;
+    int*                entryAtom;
+};
+
 template <int MODE>
-__global__ void nlbLaneKernel(int n, int numElements, int NIMG,
+__global__ void __launch_bounds__(256, 4) nlbLaneKernel(int n, int numElements, int NIMG,
                               double const* __restrict__ pos,
                               int const* __restrict__ structOf,
                               BatchStruct const* __restrict__ bs,
+                              __grid_constant__ BatchStruct const one,
                               int const* __restrict__ structAtoms,
                               int* __restrict__ nbrCount,
                               int* __restrict__ nbrCountElem,
-                              int const* __restrict__ nbrOff,
-                              unsigned long long* __restrict__ key,
+                              int const* __restrict__ nbrOff, LaneOut const out,
                               int const* __restrict__ status)
 {
     if (status[ST_FLAGS] & FLAG_ABORT) return;
     int const lane = threadIdx.x & 31;
     int const i = (int)((blockIdx.x * (long)blockDim.x + threadIdx.x) >> 5);
     if (i >= n) return;
-    BatchStruct const& S = bs[structOf[i]];
+    BatchStruct const& S = structOf ? bs[structOf[i]] : one;
     NLParams const& p = S.p;
-    int const nimg = p.nimg;
-    int const q0 = p.periodic ? p.pbc[0] : 0;
-    int const q1 = p.periodic ? p.pbc[1] : 0;
-    int const q2 = p.periodic ? p.pbc[2] : 0;
-    float a[3][3];
+    float q[3], m1, m2;
+    float a[3][3], inv[3][3], reach[3];
+    float const rcf = sqrtf((float)p.rc2);
 #pragma unroll
-    for (int r = 0; r < 3; ++r)
+    for (int k = 0; k < 3; ++k)
+    {
+        q[k] = p.periodic ? (float)p.pbc[k] : 0.0f;
+        float w = 0.0f;
 #pragma unroll
-        for (int c = 0; c < 3; ++c) a[r][c] = (float)p.box[r][c];
+        for (int c = 0; c < 3; ++c)
+        {
+            a[k][c] = (float)p.box[k][c];
+            inv[k][c] = (float)p.invbox[c][k];
+            w += inv[k][c] * inv[k][c];
+        }
+        reach[k] = rcf * sqrtf(w);
+    }
+    m1 = 2.0f * q[1] + 1.0f;
+    m2 = 2.0f * q[2] + 1.0f;
     double const ri[3] = {pos[3 * i], pos[3 * i + 1], pos[3 * i + 2]};
     // Largest image shift per component: sum_r |pbc_r a_r|.
     float shiftMax = 0.0f;
 #pragma unroll
     for (int c = 0; c < 3; ++c)
-        shiftMax = fmaxf(shiftMax, fabsf(a[0][c]) * q0 + fabsf(a[1][c]) * q1
-                                   + fabsf(a[2][c]) * q2);
-    float const rcf = sqrtf((float)p.rc2);
+        shiftMax = fmaxf(shiftMax, fabsf(a[0][c]) * q[0]
+                                   + fabsf(a[1][c]) * q[1]
+                                   + fabsf(a[2][c]) * q[2]);
     int total = 0;
     long const base = (MODE == 1) ? (long)nbrOff[i] : 0;
     for (int e = 0; e < numElements; ++e)
@@ -870,12 +931,27 @@ __global__ void nlbLaneKernel(int n, int numElements, int NIMG,
                 float const M = fmaxf(fmaxf(fabsf(d0), fabsf(d1)), fabsf(d2))
                               + shiftMax;
                 float const err = 8.0f * M * 5.9604645e-8f;
-                float const rc2f = (float)p.rc2
-                                 + fmaxf(1e-4f * (float)p.rc2,
-                                         4.0f * (6.0f * rcf * err
-                                                 + 3.0f * err * err));
-                int b0 = -q0, b1 = -q1, b2 = -q2;
-                for (int img = 0; img < nimg; ++img)
+                float const slack = fmaxf(1e-4f * (float)p.rc2,
+                                          4.0f * (6.0f * rcf * err
+                                                  + 3.0f * err * err));
+                float const above = (float)p.rc2 + slack;
+                float const below = (float)p.rc2 - slack;
+                // The images of the range one after another (one loop: its
+                // trip count is the largest number of images of a lane, not
+                // the product of the largest ranges), counters as floats.
+                float lo[3], hi[3];
+#pragma unroll
+                for (int k = 0; k < 3; ++k)
+                {
+                    float const f = d0 * inv[k][0] + d1 * inv[k][1]
+                                  + d2 * inv[k][2];
+                    float const r = reach[k] + 1e-3f + 1e-4f * fabsf(f);
+                    lo[k] = fmaxf(-q[k], ceilf(-r - f));
+                    hi[k] = fminf(q[k], floorf(r - f));
+                }
+                bool more = lo[0] <= hi[0] && lo[1] <= hi[1] && lo[2] <= hi[2];
+                float b0 = lo[0], b1 = lo[1], b2 = lo[2];
+                while (more)
                 {
                     float const x = d0 + b0 * a[0][0] + b1 * a[1][0]
                                   + b2 * a[2][0];
@@ -883,20 +959,32 @@ __global__ void nlbLaneKernel(int n, int numElements, int NIMG,
                                   + b2 * a[2][1];
                     float const z = d2 + b0 * a[0][2] + b1 * a[1][2]
                                   + b2 * a[2][2];
-                    if (x * x + y * y + z * z <= rc2f
-                        && !(j == i && b0 == 0 && b1 == 0 && b2 == 0))
+                    float const r2 = x * x + y * y + z * z;
+                    if (r2 <= above
+                        && !(j == i && b0 == 0.0f && b1 == 0.0f && b2 == 0.0f))
                     {
                         double dr[3];
-                        if (nlTest(p, ri, pos, j, b0, b1, b2, dr))
-                            mask[img >> 5] |= 1u << (img & 31);
-                    }
-                    if (++b2 > q2)
-                    {
-                        b2 = -q2;
-                        if (++b1 > q1)
+                        if (r2 < below
+                            || nlTest(p, ri, pos, j, (int)b0, (int)b1,
+                                      (int)b2, dr))
                         {
-                            b1 = -q1;
-                            ++b0;
+                            int const img = (int)(((b0 + q[0]) * m1 + b1
+                                                   + q[1]) * m2 + b2 + q[2]);
+#pragma unroll
+                            for (int w = 0; w < 4; ++w)
+                                if (img >> 5 == w) mask[w] |= 1u << (img & 31);
+                        }
+                    }
+                    b2 += 1.0f;
+                    if (b2 > hi[2])
+                    {
+                        b2 = lo[2];
+                        b1 += 1.0f;
+                        if (b1 > hi[1])
+                        {
+                            b1 = lo[1];
+                            b0 += 1.0f;
+                            more = b0 <= hi[0];
                         }
                     }
                 }
@@ -913,7 +1001,8 @@ __global__ void nlbLaneKernel(int n, int numElements, int NIMG,
             int const sum = __shfl_sync(0xffffffffu, incl, 31);
             if (MODE == 1 && c > 0)
             {
-                int off = total + incl - c;
+                long o = base + total + incl - c;
+#pragma unroll
                 for (int w = 0; w < 4; ++w)
                 {
                     unsigned m = mask[w];
@@ -921,7 +1010,23 @@ __global__ void nlbLaneKernel(int n, int numElements, int NIMG,
                     {
                         int const img = (w << 5) + __ffs(m) - 1;
                         m &= m - 1;
-                        key[base + off++] = nlKey(e, j, img, n, NIMG);
+                        int b0, b1, b2;
+                        imgDecode(p, img, b0, b1, b2);
+                        double dr[3];
+                        nlTest(p, ri, pos, j, b0, b1, b2, dr);
+                        double const n2 = __dadd_rn(
+                            __dadd_rn(__dmul_rn(dr[0], dr[0]),
+                                      __dmul_rn(dr[1], dr[1])),
+                            __dmul_rn(dr[2], dr[2]));
+                        out.key[o] = nlKey(e, j, img, n, NIMG);
+                        out.nbrIdx[o] = j;
+                        out.nbrEl[o] = (int8_t)e;
+                        out.dx[o] = dr[0];
+                        out.dy[o] = dr[1];
+                        out.dz[o] = dr[2];
+                        out.dd[o] = __dsqrt_rn(n2);
+                        out.entryAtom[o] = i;
+                        ++o;
                     }
                 }
             }
@@ -941,43 +1046,50 @@ void launchNeighborListBatch(NLBatchLaunch const& L, cudaStream_t s)
     int const gAtoms = (n + tb - 1) / tb;
     int const wpb = L.warpsPerBlock > 0 ? L.warpsPerBlock : 4;
     int const gWarp = (n + wpb - 1) / wpb;
-    nlbPrepareKernel<<<gAtoms, tb, 0, s>>>(n, L.posIn, L.structOf, L.bs,
+    nlbPrepareKernel<<<gAtoms, tb, 0, s>>>(n, L.posIn, L.structOf, L.bs, L.one,
                                            L.normalize, L.convLength, L.pos);
+    long const cap = L.capacity;
+    int const gE = (int)((cap + tb - 1) / tb);
     // Structures with more than 128 images (boxes below rc / 2) take the
     // plain brute path.
     if (L.NIMG <= 128)
     {
+        LaneOut const out{L.key, L.nbrIdx, L.nbrEl, L.dx, L.dy, L.dz, L.dd,
+                          L.entryAtom};
         nlbLaneKernel<0><<<gWarp, 32 * wpb, 0, s>>>(
-            n, L.numElements, L.NIMG, L.pos, L.structOf, L.bs,
-            L.structAtoms, L.nbrCount, L.nbrCountElem, L.nbrOff, L.key,
+            n, L.numElements, L.NIMG, L.pos, L.structOf, L.bs, L.one,
+            L.structAtoms, L.nbrCount, L.nbrCountElem, L.nbrOff, out,
             L.status);
         nlScanKernel<<<1, 1024, 0, s>>>(n, L.nbrCount, L.nbrOff, L.capacity,
                                         L.status);
         nlbLaneKernel<1><<<gWarp, 32 * wpb, 0, s>>>(
-            n, L.numElements, L.NIMG, L.pos, L.structOf, L.bs,
-            L.structAtoms, L.nbrCount, L.nbrCountElem, L.nbrOff, L.key,
+            n, L.numElements, L.NIMG, L.pos, L.structOf, L.bs, L.one,
+            L.structAtoms, L.nbrCount, L.nbrCountElem, L.nbrOff, out,
             L.status);
+        noteLaunches(5);
+        if (L.structOf)
+            nlbMirrorKernel<<<gE > 0 ? gE : 1, tb, 0, s>>>(
+                n, L.NIMG, L.elem, L.structOf, L.bs, L.nbrOff, L.key,
+                L.nbrIdx, L.entryAtom, L.mirror, L.status);
+        else
+            nlMirrorKernel<<<gE > 0 ? gE : 1, tb, 0, s>>>(
+                n, L.NIMG, L.elem, L.nbrOff, L.key, L.nbrIdx, L.entryAtom,
+                L.mirror, L.status);
+        return;
     }
-    else
-    {
-        nlbBruteKernel<0><<<gWarp, 32 * wpb, 0, s>>>(
-            n, L.numElements, L.NIMG, L.pos, L.structOf, L.bs,
-            L.structAtoms, L.nbrCount, L.nbrCountElem, L.nbrOff, L.key,
-            L.status);
-        nlScanKernel<<<1, 1024, 0, s>>>(n, L.nbrCount, L.nbrOff, L.capacity,
-                                        L.status);
-        nlbBruteKernel<1><<<gWarp, 32 * wpb, 0, s>>>(
-            n, L.numElements, L.NIMG, L.pos, L.structOf, L.bs,
-            L.structAtoms, L.nbrCount, L.nbrCountElem, L.nbrOff, L.key,
-            L.status);
-    }
+    nlbBruteKernel<0><<<gWarp, 32 * wpb, 0, s>>>(
+        n, L.numElements, L.NIMG, L.pos, L.structOf, L.bs, L.structAtoms,
+        L.nbrCount, L.nbrCountElem, L.nbrOff, L.key, L.status);
+    nlScanKernel<<<1, 1024, 0, s>>>(n, L.nbrCount, L.nbrOff, L.capacity,
+                                    L.status);
+    nlbBruteKernel<1><<<gWarp, 32 * wpb, 0, s>>>(
+        n, L.numElements, L.NIMG, L.pos, L.structOf, L.bs, L.structAtoms,
+        L.nbrCount, L.nbrCountElem, L.nbrOff, L.key, L.status);
     nlbFinishKernel<<<gWarp, 32 * wpb, 0, s>>>(
         n, L.NIMG, L.pos, L.elem, L.structOf, L.bs, L.nbrOff, L.key,
         L.nbrIdx, L.nbrEl, L.dx, L.dy, L.dz, L.dd, L.status);
     nlEntryAtomKernel<<<gAtoms, tb, 0, s>>>(n, L.nbrOff, L.entryAtom,
                                             L.status);
-    long const cap = L.capacity;
-    int const gE = (int)((cap + tb - 1) / tb);
     noteLaunches(7);
     nlbMirrorKernel<<<gE > 0 ? gE : 1, tb, 0, s>>>(
         n, L.NIMG, L.elem, L.structOf, L.bs, L.nbrOff, L.key, L.nbrIdx,
