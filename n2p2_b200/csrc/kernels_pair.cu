@@ -61,7 +61,7 @@ std::size_t layout(PairParams const& T, PairLaunch& L, int pass)
     int const ne = T.numElements;
     bool narrow = false;
     for (int e = 0; e < ne; ++e) narrow = narrow || T.narrow[e];
-    take(L.oTab, r == 8 ? 8 * sfk::kExpTableSize : 0);
+    take(L.oTab, r == 8 ? 8 * 256 : 0);    // kPairExp2
     // The tables of all elements, those of the inner loops first, while they
     // are small (the water potentials: 4 to 7 KB); else they are read
     // through L1.
@@ -92,7 +92,7 @@ std::size_t layout(PairParams const& T, PairLaunch& L, int pass)
         at = x;
         L.pairCap = std::max(512, L.cap);
         take(L.oPairs, 4 * (std::size_t)L.pairCap * w);
-        take(L.oRed, r * 16 * 33 * w);
+        take(L.oRed, r * 8 * 33 * w);
         at = std::max(at, y);
     }
     else

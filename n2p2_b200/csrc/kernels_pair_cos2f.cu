@@ -4,6 +4,6 @@
 namespace n2p2b
 {
 
-N2P2B_PAIR_LAUNCH(cos2f, float, 1, 3, (sfp2::kHasPow2), 5, 6)
+N2P2B_PAIR_LAUNCH(cos2f, float, 1, 3, (sfp2::kHasPow2), 4, 6)
 
 } // namespace n2p2b

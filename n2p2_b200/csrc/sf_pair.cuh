@@ -43,7 +43,7 @@ constexpr int kW = kT / 32;           // warps
 constexpr int kSl = 4;                // slices (lanes) per owner
 constexpr int kOw = 32 / kSl;         // owners per item
 
-constexpr double kLn64 = 0x1.62e42fefa39efp-7;     // ln2 / 64
+constexpr double kLn256 = 0x1.62e42fefa39efp-9;    // ln2 / 256
 
 template <typename R> struct V2;
 template <> struct V2<double> { using T = double2; };
@@ -71,53 +71,146 @@ struct Staged
     int           cs;         // cap + 1
 };
 
-// Series coefficients of the FP64 kernels in the constant bank: an FMA takes
-// one operand from there, while 64-bit literals cost two moves each in a loop
-// that has no registers left to keep them.
+// Polynomial coefficients of the FP64 kernels in the constant bank: an FMA
+// takes one operand from there, while 64-bit literals cost two moves each in
+// a loop that has no registers left to keep them.
+//   ex: 2^(f/256) - 1 = f (ex3 + f (ex2 + ...)), Taylor.
+//   ch, sh: cos(sqrt w) and sin(sqrt w) / sqrt w on 0 <= w <= (pi/2)^2 (r up
+//   to the cutoff), interpolated at the Chebyshev nodes; their errors there,
+//   rounding of the coefficients included, are 6.4e-17 and 1.4e-17 (a Taylor
+//   series of that error needs two terms more).
 struct PairConst
 {
-    double ex[5];      // 2^(f/64) - 1: coefficients of f^5 .. f
-    double ch[10];     // cos(sqrt w): n = 9 .. 0 terms (start n = 10)
-    double sh[10];     // sin(sqrt w) / sqrt w
-    double ch10, sh10;
-    double invL, shift;
+    double ex[4];
+    double ch[9], sh[9];
+    double shift;
 };
 __constant__ PairConst kPC = {
-    {kLn64 * kLn64 * kLn64 * kLn64 * kLn64 / 120.0,
-     kLn64 * kLn64 * kLn64 * kLn64 / 24.0, kLn64 * kLn64 * kLn64 / 6.0,
-     kLn64 * kLn64 / 2.0, kLn64},
-    {-InvFact<18>::value, InvFact<16>::value, -InvFact<14>::value,
-     InvFact<12>::value, -InvFact<10>::value, InvFact<8>::value,
-     -InvFact<6>::value, InvFact<4>::value, -InvFact<2>::value, 1.0},
-    {-InvFact<19>::value, InvFact<17>::value, -InvFact<15>::value,
-     InvFact<13>::value, -InvFact<11>::value, InvFact<9>::value,
-     -InvFact<7>::value, InvFact<5>::value, -InvFact<3>::value, 1.0},
-    InvFact<20>::value, InvFact<21>::value, -0x1.71547652b82fep+6, 0x1.8p52};
+    {kLn256 * kLn256 * kLn256 * kLn256 / 24.0, kLn256 * kLn256 * kLn256 / 6.0,
+     kLn256 * kLn256 / 2.0, kLn256},
+    {0x1.9f237664fdb61p-45, -0x1.9350a15519b35p-37, 0x1.1eecdf2eb6420p-29,
+     -0x1.27e4f97908e2ep-22, 0x1.a01a01994b814p-16, -0x1.6c16c16c09b34p-10,
+     0x1.55555555553c4p-5, -0x1.ffffffffffffbp-2, 1.0},
+    {0x1.88382132048bcp-49, -0x1.ae439c8976ed0p-41, 0x1.6123ccd07d338p-33,
+     -0x1.ae6454d052da4p-26, 0x1.71de3a528cce3p-19, -0x1.a01a01a0147e9p-13,
+     0x1.11111111110bcp-7, -0x1.5555555555555p-3, 1.0},
+    0x1.8p52};
+
+// 2^(j / 256), rounded to nearest; staged into shared memory.
+constexpr int kPairExpSize = 256;
+static __device__ double const kPairExp2[kPairExpSize] = {
+    0x1.0000000000000p+0, 0x1.00b1afa5abcbfp+0, 0x1.0163da9fb3335p+0,
+    0x1.02168143b0281p+0, 0x1.02c9a3e778061p+0, 0x1.037d42e11bbccp+0,
+    0x1.04315e86e7f85p+0, 0x1.04e5f72f654b1p+0, 0x1.059b0d3158574p+0,
+    0x1.0650a0e3c1f89p+0, 0x1.0706b29ddf6dep+0, 0x1.07bd42b72a836p+0,
+    0x1.0874518759bc8p+0, 0x1.092bdf66607e0p+0, 0x1.09e3ecac6f383p+0,
+    0x1.0a9c79b1f3919p+0, 0x1.0b5586cf9890fp+0, 0x1.0c0f145e46c85p+0,
+    0x1.0cc922b7247f7p+0, 0x1.0d83b23395decp+0, 0x1.0e3ec32d3d1a2p+0,
+    0x1.0efa55fdfa9c5p+0, 0x1.0fb66affed31bp+0, 0x1.1073028d7233ep+0,
+    0x1.11301d0125b51p+0, 0x1.11edbab5e2ab6p+0, 0x1.12abdc06c31ccp+0,
+    0x1.136a814f204abp+0, 0x1.1429aaea92de0p+0, 0x1.14e95934f312ep+0,
+    0x1.15a98c8a58e51p+0, 0x1.166a45471c3c2p+0, 0x1.172b83c7d517bp+0,
+    0x1.17ed48695bbc0p+0, 0x1.18af9388c8deap+0, 0x1.1972658375d2fp+0,
+    0x1.1a35beb6fcb75p+0, 0x1.1af99f8138a1cp+0, 0x1.1bbe084045cd4p+0,
+    0x1.1c82f95281c6bp+0, 0x1.1d4873168b9aap+0, 0x1.1e0e75eb44027p+0,
+    0x1.1ed5022fcd91dp+0, 0x1.1f9c18438ce4dp+0, 0x1.2063b88628cd6p+0,
+    0x1.212be3578a819p+0, 0x1.21f49917ddc96p+0, 0x1.22bdda27912d1p+0,
+    0x1.2387a6e756238p+0, 0x1.2451ffb82140ap+0, 0x1.251ce4fb2a63fp+0,
+    0x1.25e85711ece75p+0, 0x1.26b4565e27cddp+0, 0x1.2780e341ddf29p+0,
+    0x1.284dfe1f56381p+0, 0x1.291ba7591bb70p+0, 0x1.29e9df51fdee1p+0,
+    0x1.2ab8a66d10f13p+0, 0x1.2b87fd0dad990p+0, 0x1.2c57e39771b2fp+0,
+    0x1.2d285a6e4030bp+0, 0x1.2df961f641589p+0, 0x1.2ecafa93e2f56p+0,
+    0x1.2f9d24abd886bp+0, 0x1.306fe0a31b715p+0, 0x1.31432edeeb2fdp+0,
+    0x1.32170fc4cd831p+0, 0x1.32eb83ba8ea32p+0, 0x1.33c08b26416ffp+0,
+    0x1.3496266e3fa2dp+0, 0x1.356c55f929ff1p+0, 0x1.36431a2de883bp+0,
+    0x1.371a7373aa9cbp+0, 0x1.37f26231e754ap+0, 0x1.38cae6d05d866p+0,
+    0x1.39a401b7140efp+0, 0x1.3a7db34e59ff7p+0, 0x1.3b57fbfec6cf4p+0,
+    0x1.3c32dc313a8e5p+0, 0x1.3d0e544ede173p+0, 0x1.3dea64c123422p+0,
+    0x1.3ec70df1c5175p+0, 0x1.3fa4504ac801cp+0, 0x1.40822c367a024p+0,
+    0x1.4160a21f72e2ap+0, 0x1.423fb2709468ap+0, 0x1.431f5d950a897p+0,
+    0x1.43ffa3f84b9d4p+0, 0x1.44e086061892dp+0, 0x1.45c2042a7d232p+0,
+    0x1.46a41ed1d0057p+0, 0x1.4786d668b3237p+0, 0x1.486a2b5c13cd0p+0,
+    0x1.494e1e192aed2p+0, 0x1.4a32af0d7d3dep+0, 0x1.4b17dea6db7d7p+0,
+    0x1.4bfdad5362a27p+0, 0x1.4ce41b817c114p+0, 0x1.4dcb299fddd0dp+0,
+    0x1.4eb2d81d8abffp+0, 0x1.4f9b2769d2ca7p+0, 0x1.508417f4531eep+0,
+    0x1.516daa2cf6642p+0, 0x1.5257de83f4eefp+0, 0x1.5342b569d4f82p+0,
+    0x1.542e2f4f6ad27p+0, 0x1.551a4ca5d920fp+0, 0x1.56070dde910d2p+0,
+    0x1.56f4736b527dap+0, 0x1.57e27dbe2c4cfp+0, 0x1.58d12d497c7fdp+0,
+    0x1.59c0827ff07ccp+0, 0x1.5ab07dd485429p+0, 0x1.5ba11fba87a03p+0,
+    0x1.5c9268a5946b7p+0, 0x1.5d84590998b93p+0, 0x1.5e76f15ad2148p+0,
+    0x1.5f6a320dceb71p+0, 0x1.605e1b976dc09p+0, 0x1.6152ae6cdf6f4p+0,
+    0x1.6247eb03a5585p+0, 0x1.633dd1d1929fdp+0, 0x1.6434634ccc320p+0,
+    0x1.652b9febc8fb7p+0, 0x1.6623882552225p+0, 0x1.671c1c70833f6p+0,
+    0x1.68155d44ca973p+0, 0x1.690f4b19e9538p+0, 0x1.6a09e667f3bcdp+0,
+    0x1.6b052fa75173ep+0, 0x1.6c012750bdabfp+0, 0x1.6cfdcddd47645p+0,
+    0x1.6dfb23c651a2fp+0, 0x1.6ef9298593ae5p+0, 0x1.6ff7df9519484p+0,
+    0x1.70f7466f42e87p+0, 0x1.71f75e8ec5f74p+0, 0x1.72f8286ead08ap+0,
+    0x1.73f9a48a58174p+0, 0x1.74fbd35d7cbfdp+0, 0x1.75feb564267c9p+0,
+    0x1.77024b1ab6e09p+0, 0x1.780694fde5d3fp+0, 0x1.790b938ac1cf6p+0,
+    0x1.7a11473eb0187p+0, 0x1.7b17b0976cfdbp+0, 0x1.7c1ed0130c132p+0,
+    0x1.7d26a62ff86f0p+0, 0x1.7e2f336cf4e62p+0, 0x1.7f3878491c491p+0,
+    0x1.80427543e1a12p+0, 0x1.814d2add106d9p+0, 0x1.82589994cce13p+0,
+    0x1.8364c1eb941f7p+0, 0x1.8471a4623c7adp+0, 0x1.857f4179f5b21p+0,
+    0x1.868d99b4492edp+0, 0x1.879cad931a436p+0, 0x1.88ac7d98a6699p+0,
+    0x1.89bd0a478580fp+0, 0x1.8ace5422aa0dbp+0, 0x1.8be05bad61778p+0,
+    0x1.8cf3216b5448cp+0, 0x1.8e06a5e0866d9p+0, 0x1.8f1ae99157736p+0,
+    0x1.902fed0282c8ap+0, 0x1.9145b0b91ffc6p+0, 0x1.925c353aa2fe2p+0,
+    0x1.93737b0cdc5e5p+0, 0x1.948b82b5f98e5p+0, 0x1.95a44cbc8520fp+0,
+    0x1.96bdd9a7670b3p+0, 0x1.97d829fde4e50p+0, 0x1.98f33e47a22a2p+0,
+    0x1.9a0f170ca07bap+0, 0x1.9b2bb4d53fe0dp+0, 0x1.9c49182a3f090p+0,
+    0x1.9d674194bb8d5p+0, 0x1.9e86319e32323p+0, 0x1.9fa5e8d07f29ep+0,
+    0x1.a0c667b5de565p+0, 0x1.a1e7aed8eb8bbp+0, 0x1.a309bec4a2d33p+0,
+    0x1.a42c980460ad8p+0, 0x1.a5503b23e255dp+0, 0x1.a674a8af46052p+0,
+    0x1.a799e1330b358p+0, 0x1.a8bfe53c12e59p+0, 0x1.a9e6b5579fdbfp+0,
+    0x1.ab0e521356ebap+0, 0x1.ac36bbfd3f37ap+0, 0x1.ad5ff3a3c2774p+0,
+    0x1.ae89f995ad3adp+0, 0x1.afb4ce622f2ffp+0, 0x1.b0e07298db666p+0,
+    0x1.b20ce6c9a8952p+0, 0x1.b33a2b84f15fbp+0, 0x1.b468415b749b1p+0,
+    0x1.b59728de5593ap+0, 0x1.b6c6e29f1c52ap+0, 0x1.b7f76f2fb5e47p+0,
+    0x1.b928cf22749e4p+0, 0x1.ba5b030a1064ap+0, 0x1.bb8e0b79a6f1fp+0,
+    0x1.bcc1e904bc1d2p+0, 0x1.bdf69c3f3a207p+0, 0x1.bf2c25bd71e09p+0,
+    0x1.c06286141b33dp+0, 0x1.c199bdd85529cp+0, 0x1.c2d1cd9fa652cp+0,
+    0x1.c40ab5fffd07ap+0, 0x1.c544778fafb22p+0, 0x1.c67f12e57d14bp+0,
+    0x1.c7ba88988c933p+0, 0x1.c8f6d9406e7b5p+0, 0x1.ca3405751c4dbp+0,
+    0x1.cb720dcef9069p+0, 0x1.ccb0f2e6d1675p+0, 0x1.cdf0b555dc3fap+0,
+    0x1.cf3155b5bab74p+0, 0x1.d072d4a07897cp+0, 0x1.d1b532b08c968p+0,
+    0x1.d2f87080d89f2p+0, 0x1.d43c8eacaa1d6p+0, 0x1.d5818dcfba487p+0,
+    0x1.d6c76e862e6d3p+0, 0x1.d80e316c98398p+0, 0x1.d955d71ff6075p+0,
+    0x1.da9e603db3285p+0, 0x1.dbe7cd63a8315p+0, 0x1.dd321f301b460p+0,
+    0x1.de7d5641c0658p+0, 0x1.dfc97337b9b5fp+0, 0x1.e11676b197d17p+0,
+    0x1.e264614f5a129p+0, 0x1.e3b333b16ee12p+0, 0x1.e502ee78b3ff6p+0,
+    0x1.e653924676d76p+0, 0x1.e7a51fbc74c83p+0, 0x1.e8f7977cdb740p+0,
+    0x1.ea4afa2a490dap+0, 0x1.eb9f4867cca6ep+0, 0x1.ecf482d8e67f1p+0,
+    0x1.ee4aaa2188510p+0, 0x1.efa1bee615a27p+0, 0x1.f0f9c1cb6412ap+0,
+    0x1.f252b376bba97p+0, 0x1.f3ac948dd7274p+0, 0x1.f50765b6e4540p+0,
+    0x1.f6632798844f8p+0, 0x1.f7bfdad9cbe14p+0, 0x1.f91d802243c89p+0,
+    0x1.fa7c1819e90d8p+0, 0x1.fbdba3692d514p+0, 0x1.fd3c22b8f71f1p+0,
+    0x1.fe9d96b2a23d9p+0,
+};
 
 // Constants of one run: eta in the exponential's unit.
-//   FP64: exp(-eta s) = 2^(k/64) 2^(f/64), k = rint(y), f = y - k with
-//   y = -eta s 64/ln2; f is formed by one fma from s (no product rounding),
-//   2^(f/64) - 1 by its Taylor polynomial of degree 5 in f (|f| <= 1/2:
-//   truncation below 4e-17), 2^(j/64) from the table.  The error is that of
+//   FP64: exp(-eta s) = 2^(k/256) 2^(f/256), k = rint(y), f = y - k with
+//   y = -eta s 256/ln2; f is formed by one fma from s (no product rounding),
+//   2^(f/256) - 1 by its Taylor polynomial of degree 4 in f (|f| <= 1/2:
+//   truncation below 4e-17), 2^(j/256) from the table.  The error is that of
 //   y's factor, |eta s| 2^-53, and 1 ulp, as for exp of the rounded
 //   product.  Results below 2^-1020 stay near 2^-1020.
 __device__ __forceinline__ double expScale(double eta)
 {
-    return eta * -0x1.71547652b82fep+6;
+    return eta * -0x1.71547652b82fep+8;
 }
 __device__ __forceinline__ double expScaled(double e2, double s,
                                             double const* tab)
 {
     double const t = fma(s, e2, kPC.shift);
-    int const k = max(__double2loint(t), -64 * 1020);
+    int const k = max(__double2loint(t), -256 * 1020);
     double const f = fma(s, e2, kPC.shift - t);
     double p = fma(f, kPC.ex[0], kPC.ex[1]);
-#pragma unroll
-    for (int n = 2; n < 5; ++n) p = fma(p, f, kPC.ex[n]);
+    p = fma(p, f, kPC.ex[2]);
+    p = fma(p, f, kPC.ex[3]);
     double const q = p * f;
-    double const tj = tab[k & (kExpTableSize - 1)];
+    double const tj = tab[k & (kPairExpSize - 1)];
     double const tm = __hiloint2double(
-        __double2hiint(tj) + ((k >> 6) << 20), __double2loint(tj));
+        __double2hiint(tj) + ((k >> 8) << 20), __double2loint(tj));
     return fma(tm, q, tm);
 }
 __device__ __forceinline__ float expScale(float eta)
@@ -134,49 +227,40 @@ __device__ __forceinline__ float expScaled(float e2, float s, double const*)
 template <typename R>
 __device__ __forceinline__ R expUnscale()
 {
-    return sizeof(R) == 8 ? R(-0x1.62e42fefa39efp-7) : R(-0.693147181f);
+    return sizeof(R) == 8 ? R(-0x1.62e42fefa39efp-9) : R(-0.693147181f);
 }
 
-template <typename R, int N, int K>
-struct SeriesR
-{
-    __device__ static __forceinline__ R run(R v, R acc)
-    {
-        constexpr double c = ((N & 1) ? -1.0 : 1.0) * InvFact<2 * N + K>::value;
-        return SeriesR<R, N - 1, K>::run(v, fma(acc, v, R(c)));
-    }
-};
-template <typename R, int K>
-struct SeriesR<R, -1, K>
-{
-    __device__ static __forceinline__ R run(R, R acc) { return acc; }
-};
-
-// cos and sin(x)/x of the half angle from w = (a r / 2)^2 <= pi^2 / 4: FP64
-// as halfAngleCosSinc; FP32 with the terms up to n = 6 (first omitted terms
-// 6.5e-9 and 4.3e-10 relative to 1).
+// cos and sin(x)/x of the half angle from w = (a r / 2)^2.  FP32: degrees 5
+// and 4, interpolated likewise (errors 2.8e-8 and 8.2e-9).
 __device__ __forceinline__ double halfAngleCos(double w)
 {
-    double c = kPC.ch10;
+    double c = kPC.ch[0];
 #pragma unroll
-    for (int n = 0; n < 10; ++n) c = fma(c, w, kPC.ch[n]);
+    for (int n = 1; n < 9; ++n) c = fma(c, w, kPC.ch[n]);
     return c;
 }
 __device__ __forceinline__ void halfAngle(double w, double& ch, double& sh)
 {
     ch = halfAngleCos(w);
-    sh = kPC.sh10;
+    sh = kPC.sh[0];
 #pragma unroll
-    for (int n = 0; n < 10; ++n) sh = fma(sh, w, kPC.sh[n]);
-}
-__device__ __forceinline__ void halfAngle(float w, float& ch, float& sh)
-{
-    ch = SeriesR<float, 5, 0>::run(w, (float)InvFact<12>::value);
-    sh = SeriesR<float, 5, 1>::run(w, (float)InvFact<13>::value);
+    for (int n = 1; n < 9; ++n) sh = fma(sh, w, kPC.sh[n]);
 }
 __device__ __forceinline__ float halfAngleCos(float w)
 {
-    return SeriesR<float, 5, 0>::run(w, (float)InvFact<12>::value);
+    float c = fmaf(w, -2.605053911e-07f, 2.476010310e-05f);
+    c = fmaf(c, w, -1.388836016e-03f);
+    c = fmaf(c, w, 4.166663615e-02f);
+    c = fmaf(c, w, -4.999999936e-01f);
+    return fmaf(c, w, 1.0f);
+}
+__device__ __forceinline__ void halfAngle(float w, float& ch, float& sh)
+{
+    ch = halfAngleCos(w);
+    float s = fmaf(w, 2.605095804e-06f, -1.980901230e-04f);
+    s = fmaf(s, w, 8.333050103e-03f);
+    s = fmaf(s, w, -1.666665795e-01f);
+    sh = fmaf(s, w, 9.999999957e-01f);
 }
 
 // f_c(r_jk) and, with DERIV, q = f_c'(r_jk) / r_jk.  CT = 1 is the cosine
@@ -363,6 +447,21 @@ __device__ __forceinline__ unsigned maskWord(float4 const* pos, int t, int q,
     }
     if (a.w != 0.0f) m = 0u;
     if (cnt - (q << 5) < 32) m &= (1u << (cnt & 31)) - 1u;
+    return m;
+}
+
+// Transpose of the 32 x 32 bit matrix whose row l is lane l's word.
+__device__ __forceinline__ unsigned transpose32(unsigned m, int lane)
+{
+    unsigned keep = 0x0000ffffu;
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1)
+    {
+        unsigned const v = __shfl_xor_sync(kFull, m, d);
+        m = (lane & d) ? ((m & ~keep) | ((v & ~keep) >> d))
+                       : ((m & keep) | ((v & keep) << d));
+        keep ^= keep << (d >> 1);
+    }
     return m;
 }
 
@@ -616,8 +715,8 @@ __device__ __forceinline__ void stageExpTable(unsigned char* sm,
     if (sizeof(R) == 8)
     {
         double* tab = reinterpret_cast<double*>(sm + L.oTab);
-        for (int j = threadIdx.x; j < kExpTableSize; j += kT)
-            tab[j] = kExp2Table[j];
+        for (int j = threadIdx.x; j < kPairExpSize; j += kT)
+            tab[j] = kPairExp2[j];
     }
 }
 
@@ -636,7 +735,7 @@ struct Walk
     Staged<R> W;
     unsigned const* bits; // [t][words], k > t
     unsigned* pairs;      // the warp's pair list [pairCap]
-    R*        red;        // 16 x 33 lane sums
+    R*        red;        // 8 x 33 lane sums
     R*        Gp;         // the warp's sums [maxSF]
     PairCell const* cells;
     int       words, pairCap, b1, x1, b2, x2, same, lane, warp, warps;
@@ -717,28 +816,30 @@ __device__ __forceinline__ void walkPairs(Walk<R> const& w, F&& f)
     }
 }
 
-// Adds the lanes' sums of N cells to the warp's values: sixteen cells at a
-// time, lane (row, half) adds sixteen lanes of its cell, then its neighbor.
+// Adds the lanes' sums of N cells to the warp's values: eight cells at a
+// time through shared memory, lane (row, quarter) adds eight lanes of its
+// cell, then the quarters are added.
 template <typename R, int N>
 __device__ __forceinline__ void flushCells(Walk<R> const& w, R const (&acc)[N],
                                            int cell0, int cells)
 {
 #pragma unroll
-    for (int c0 = 0; c0 < N; c0 += 16)
+    for (int c0 = 0; c0 < N; c0 += 8)
     {
         if (c0 < cells)
         {
 #pragma unroll
-            for (int c = 0; c < 16; ++c)
+            for (int c = 0; c < 8; ++c)
                 if (c0 + c < N) w.red[c * 33 + w.lane] = acc[c0 + c];
             __syncwarp();
-            int const row = w.lane >> 1;
+            int const row = w.lane >> 2;
             R v = R(0);
 #pragma unroll
-            for (int q = 0; q < 16; ++q)
-                v += w.red[row * 33 + (w.lane & 1) * 16 + q];
+            for (int q = 0; q < 8; ++q)
+                v += w.red[row * 33 + (w.lane & 3) * 8 + q];
             v += __shfl_xor_sync(kFull, v, 1);
-            if ((w.lane & 1) == 0 && c0 + row < cells)
+            v += __shfl_xor_sync(kFull, v, 2);
+            if ((w.lane & 3) == 0 && c0 + row < cells)
             {
                 int const sf = w.cells[cell0 + c0 + row].sf;
                 if (sf >= 0) w.Gp[sf] += v;
@@ -1035,7 +1136,7 @@ pairValueKernel(__grid_constant__ SFParams const P,
     w.bits = bits;
     w.pairs = reinterpret_cast<unsigned*>(mine + L.oPairs) + L.pairCap * warp;
     w.pairCap = L.pairCap;
-    w.red = reinterpret_cast<R*>(mine + L.oRed) + warp * 16 * 33;
+    w.red = reinterpret_cast<R*>(mine + L.oRed) + warp * 8 * 33;
     w.Gp = Gp + warp * maxSF;
     w.lane = lane;
     w.warp = warp;
@@ -1242,6 +1343,9 @@ __device__ __forceinline__ void pow2Forces(SFParams const& P,
     unsigned const mask = MASK ? (unsigned)MASK : u.mask;
     R al = R(0), vx = R(0), vy = R(0), vz = R(0);
     P2 const* const C2 = reinterpret_cast<P2 const*>(C);
+    R h1[NR];             // zeta = 1: d/dcos is a constant
+#pragma unroll
+    for (int a = 0; a < NR; ++a) h1[a] = C2[a].y - C2[a].x;
 #pragma unroll 1
     for (int st = 0; st < p.steps; ++st)
     {
@@ -1278,8 +1382,8 @@ __device__ __forceinline__ void pow2Forces(SFParams const& P,
                     P2 const c = C2[z * NR + a];
                     b[a] = z == 0 ? c.x * Pm : b[a] + c.x * Pm;
                     b[a] += c.y * Pp;
-                    h[a] = z == 0 ? c.y : h[a] + c.y * hp;
-                    h[a] = z == 0 ? h[a] - c.x : h[a] - c.x * hm;
+                    if (z == 0) h[a] = h1[a];
+                    else h[a] = (h[a] + c.y * hp) - c.x * hm;
                 }
             }
             else if (z == 0)
@@ -1709,36 +1813,47 @@ pairTermKernel(__grid_constant__ SFParams const P,
         stageAtom<R, CT, WPA, true>(P, T, L, h, tm, pos, (R*)nullptr, arad, C,
                                     tb.q, W);
         Tm::sync();
-        // Validity masks (narrow units), lanes own rows; with them per row the
-        // partners of the elements below each one and in all, and the key
-        // that orders the owners.
+        // Validity masks (narrow units): (32 rows, word) blocks on and above
+        // the diagonal, those below are their transposes.
         if (anyNarrow)
         {
             float const rc2 = maskRc2(T, ec, sizeof(R) == 8);
             int const nb = (cnt + 31) >> 5;
-            for (int rb = warp; rb < nb; rb += WPA)
+            int task = 0;
+            for (int rb = 0; rb < nb; ++rb)
+                for (int q = rb; q < nb; ++q)
+                {
+                    if ((task++ & (WPA - 1)) != warp) continue;
+                    int const t = (rb << 5) + lane;
+                    unsigned m = maskWord(pos, t, q, cnt, rc2);
+                    if (q == rb)
+                    {
+                        m &= ~(1u << lane);
+                        if (t < cnt) bits[t * words + q] = m;
+                        continue;
+                    }
+                    bits[t * words + q] = m;
+                    m = transpose32(m, lane);
+                    int const u = (q << 5) + lane;
+                    if (u < cnt) bits[u * words + rb] = m;
+                }
+            Tm::sync();
+            // Per row the partners of the elements below each one and in
+            // all, and the key that orders the owners.
+            for (int t = tm.tid; t < cnt; t += Tm::kThreads)
             {
-                int const t = (rb << 5) + lane;
-                bool const in = t < cnt;
                 int total = 0, e = 0;
                 for (int q = 0; q < nb; ++q)
                 {
-                    unsigned m = maskWord(pos, t, q, cnt, rc2);
-                    if (q == rb) m &= ~(1u << lane);
-                    if (in) bits[t * words + q] = m;
+                    unsigned const m = bits[t * words + q];
                     for (; e < ne && h.eb[e] < (q + 1) << 5; ++e)
-                        if (in)
-                            pre[t * (ne + 1) + e] = (unsigned short)(
-                                total
-                                + __popc(m & ((1u << (h.eb[e] & 31)) - 1u)));
+                        pre[t * (ne + 1) + e] = (unsigned short)(
+                            total + __popc(m & ((1u << (h.eb[e] & 31)) - 1u)));
                     total += __popc(m);
                 }
-                if (in)
-                {
-                    for (; e <= ne; ++e)
-                        pre[t * (ne + 1) + e] = (unsigned short)total;
-                    key[t] = ((unsigned)total << 16) | (0xffffu - (unsigned)t);
-                }
+                for (; e <= ne; ++e)
+                    pre[t * (ne + 1) + e] = (unsigned short)total;
+                key[t] = ((unsigned)total << 16) | (0xffffu - (unsigned)t);
             }
         }
         Tm::sync();
