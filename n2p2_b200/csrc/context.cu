@@ -381,7 +381,7 @@ struct n2p2b_context
     long         capacity = 0;
     DevBuf       keyTmp, key, nbrIdx, nbrEl, dx, dy, dz, dd, entryAtom, mirror;
     DevBuf       pairF, dGdr;
-    DevBuf       G, dEdG, dGdrSelf, Ei, selfF, F, energyOut, status;
+    DevBuf       G, Gother, dEdG, dGdrSelf, Ei, selfF, F, energyOut, status;
     int*         statusHost = nullptr;
     double*      energyHost = nullptr;
     int          sfCap = 0;      // 0 = size from the next neighbor list
@@ -480,7 +480,8 @@ struct n2p2b_context
                           &cellStart, &cellAtoms, &cellStatus, &nbrCount,
                           &nbrCountElem, &nbrOff, &keyTmp, &key, &nbrIdx,
                           &nbrEl, &dx, &dy, &dz, &dd, &entryAtom, &mirror,
-                          &pairF, &dGdr, &G, &dEdG, &dGdrSelf, &Ei, &selfF,
+                          &pairF, &dGdr, &G, &Gother, &dEdG, &dGdrSelf, &Ei,
+                          &selfF,
                           &F, &energyOut, &status, &tabGroupsDev,
                           &tabMembersDev, &pairTabs})
             b->release();
@@ -1441,20 +1442,10 @@ struct n2p2b_context
     void requireDGdr()
     {
         if (haveDGdr) return;
-        DevBuf scratch;
-        try
-        {
-            scratch.ensure(realBytes() * n * maxSF);
-            enqueueStoredSF(true, scratch.p);
-            checkLaunch("symmetry-function derivatives");
-            ck(cudaStreamSynchronize(stream), "synchronize");
-        }
-        catch (...)
-        {
-            scratch.release();
-            throw;
-        }
-        scratch.release();
+        Gother.ensure(realBytes() * n * maxSF);
+        enqueueStoredSF(true, Gother.p);
+        checkLaunch("symmetry-function derivatives");
+        ck(cudaStreamSynchronize(stream), "synchronize");
         haveDGdr = true;
     }
 
@@ -1986,6 +1977,22 @@ struct n2p2b_context
         R.scale = sfScale.as<SFScale>();
         R.range = stu.dRange.as<Range>();
         launchStudentRange(R, stream);
+        if (pairUsable())
+        {
+            // The values of the other route differ in rounding: the range
+            // holds for both, so that no atom of a training frame is gated
+            // whichever computes its symmetry functions later.
+            Gother.ensure(realBytes() * n * maxSF);
+            if (haveDGdr)
+            {
+                PairLaunch L = pairLaunch();
+                L.G = Gother.p;
+                launchPair(0, sfp, pt.p, ptDev, L, stream);
+            }
+            else enqueueStoredSF(false, Gother.p);
+            R.G = Gother.p;
+            launchStudentRange(R, stream);
+        }
         checkLaunch("training range");
         stu.haveRange = true;
     }
