@@ -77,8 +77,15 @@ std::size_t layout(PairParams const& T, PairLaunch& L, int pass)
     std::size_t const w = (std::size_t)L.wpa;
     take(L.oRec, 6 * r * cs);
     take(L.oFc, r * cs * std::max(T.maxFc - 1, 0));
-    take(L.oRad, 2 * r * cs * T.maxRad);
+    take(L.oRad, (pass == 0 ? 1 : 2) * r * cs * T.maxRad);
     if (narrow) take(L.oBits, 4 * cap * words);
+    bool sorted = false;
+    for (int e = 0; e < ne; ++e) sorted = sorted || T.sorted[e];
+    if (sorted)
+    {
+        take(L.oSort, 4 * cap);
+        if (pass == 1) take(L.oOrig, 2 * cap);
+    }
     if (pass == 0)
     {
         take(L.oG, r * w * L.maxSF);

@@ -65,8 +65,8 @@ struct Staged
     Rec<R>*       rec;        // [cs]
     R*            fc;         // [fc slot - 1][cs]: f_c (x Z)
     R*            dfc;        // [fc slot][cs]: f_c'/r (x Z)
-    R*            rad;        // [rad slot][2][cs]: window function, its
-                              // derivative / r (x Z)
+    R*            rad;        // [rad slot][cs] window functions (x Z); forces:
+                              // [rad slot][2][cs] with derivative / r
     double const* tab;        // exponential table
     int           cs;         // cap + 1
 };
@@ -503,37 +503,57 @@ __device__ __forceinline__ void stageAtom(SFParams const& P,
                                           Team<WPA> const& tm, float4* pos,
                                           R* dist, R* arad, R const* C,
                                           PairRadial const* radials,
+                                          unsigned short* orig,
+                                          unsigned* sort,
                                           Staged<R> const& S)
 {
+    bool const sorted = T.sorted[h.ec] != 0;
+    if (sorted)
+    {
+        // Keys that order the neighbors of an element by distance.
+        for (int t = tm.tid; t < h.cnt; t += Team<WPA>::kThreads)
+            sort[t] = __float_as_uint((float)L.dd[h.beg + t]);
+        Team<WPA>::sync();
+    }
     int const cs = S.cs, cnt = h.cnt, ec = h.ec;
     int const nf = T.fcBeg[ec + 1] - T.fcBeg[ec];
     int const nrad = T.radBeg[ec + 1] - T.radBeg[ec];
-    for (int t = tm.tid; t <= cnt; t += Team<WPA>::kThreads)
+    for (int e = tm.tid; e <= cnt; e += Team<WPA>::kThreads)
     {
+        int t = e;                  // place of entry e
         if (t == cnt)
         {
             R const far = R(T.farAway);
             S.rec[t] = Rec<R>{far, R(0), R(0), R(1) / far, R(0), far * far};
             for (int f = 1; f < nf; ++f) S.fc[(f - 1) * cs + t] = R(0);
-            for (int f = 0; f < 2 * nrad; ++f) S.rad[f * cs + t] = R(0);
+            for (int f = 0; f < (DERIV ? 2 : 1) * nrad; ++f)
+                S.rad[f * cs + t] = R(0);
             break;
         }
-        double const d = L.dd[h.beg + t];
+        double const d = L.dd[h.beg + e];
         R const r = R(d), ir = R(1.0 / d);
-        R const x = R(L.dx[h.beg + t]), y = R(L.dy[h.beg + t]),
-                z = R(L.dz[h.beg + t]);
+        R const x = R(L.dx[h.beg + e]), y = R(L.dy[h.beg + e]),
+                z = R(L.dz[h.beg + e]);
+        int el = 0;
+        if (DERIV || T.anyWeighted || sorted)
+            while (e >= h.eb[el + 1]) ++el;
+        if (sorted)
+        {
+            unsigned const mine = sort[e];
+            t = h.eb[el];
+            int const q1 = h.eb[el + 1];
+#pragma unroll 4
+            for (int q = h.eb[el]; q < q1; ++q)
+                t += (sort[q] < mine || (sort[q] == mine && q < e)) ? 1 : 0;
+            if (DERIV) orig[t] = (unsigned short)e;
+        }
         R const r2 = x * x + y * y + z * z;
         // Neighbors beyond the narrow cutoff are nobody's partners.
         pos[t] = (float)r2 < maskRc2(T, ec, sizeof(R) == 8)
             ? make_float4((float)x, (float)y, (float)z, 0.0f)
             : make_float4(1e18f, 0.0f, 0.0f, 1.0f);
-        R Z = R(1), f0 = R(0);
-        int el = 0;
-        if (DERIV || T.anyWeighted)
-        {
-            while (t >= h.eb[el + 1]) ++el;
-            Z = R(P.atomicNumber[el]);
-        }
+        R f0 = R(0);
+        R const Z = T.anyWeighted ? R(P.atomicNumber[el]) : R(1);
         R df0 = R(0);
         for (int f = 0; f < nf; ++f)
         {
@@ -555,8 +575,8 @@ __device__ __forceinline__ void stageAtom(SFParams const& P,
                 compactFdf<R>(w.core, w.asym != 0, R(w.center), R(w.scale), r,
                               R(P.E), v, dv);
             if (w.weighted) { v *= Z; dv *= Z; }
-            S.rad[(2 * f) * cs + t] = v;
-            S.rad[(2 * f + 1) * cs + t] = dv * ir;
+            S.rad[(DERIV ? 2 * f : f) * cs + t] = v;
+            if (DERIV) S.rad[(2 * f + 1) * cs + t] = dv * ir;
         }
         if (!DERIV) continue;
         R al = R(0), fc = R(0), dfc = R(0), ZZ = R(1);
@@ -617,11 +637,40 @@ __device__ __forceinline__ void genShapes(int ns, PairShape const* sh, R c,
 }
 
 // Window functions of theta of a compact unit, with DERIV their derivatives.
+// The usual case, all of one unit p2, runs without branches.
 template <typename R, bool DERIV>
-__device__ __forceinline__ void compShapes(SFParams const& P, int ns,
+__device__ __forceinline__ void compShapes(SFParams const& P,
+                                           PairUnit const& un,
                                            PairShape const* sh, R theta,
                                            R* phi, R* psi)
 {
+    int const ns = un.ns;
+    if (un.core == CC_POLY2)
+    {
+#pragma unroll
+        for (int s = 0; s < kPairCompShapes; ++s)
+        {
+            phi[s] = R(0);
+            if (DERIV) psi[s] = R(0);
+            if (s < ns)
+            {
+                R const sc = R(sh[s].scale);
+                R const v = (theta - R(sh[s].center)) * sc;
+                R const x = v < R(0) ? -v : v;
+                R const f = ((R(15) - R(6) * x) * x - R(10)) * (x * x * x)
+                          + R(1);
+                phi[s] = x < R(1) ? f : R(0);
+                if (DERIV)
+                {
+                    // d/dx = -30 x^2 (1 - x)^2, times the sign of v.
+                    R const y = x - x * x;
+                    R const d = (v * (R(1) - x)) * y;
+                    psi[s] = x < R(1) ? (R(-30) * sc) * d : R(0);
+                }
+            }
+        }
+        return;
+    }
 #pragma unroll
     for (int s = 0; s < kPairCompShapes; ++s)
     {
@@ -1043,7 +1092,7 @@ __device__ __forceinline__ void compactValues(SFParams const& P,
     R acc[N];
 #pragma unroll
     for (int c = 0; c < N; ++c) acc[c] = R(0);
-    int const ns = u.ns, nr = u.nr, cs = w.W.cs;
+    int const nr = u.nr, cs = w.W.cs;
     PairRun const* const runs = tb.r + u.run;
     PairShape const* const sh = tb.s + u.shape;
     walkPairs<R, NARROW>(w, [&](int tt, int kk) {
@@ -1051,7 +1100,7 @@ __device__ __forceinline__ void compactValues(SFParams const& P,
         R const c = (A.x * B.x + A.y * B.y + A.z * B.z) * (A.ir * B.ir);
         bool const ok = c > R(-1) && c < R(1);
         R phi[S];
-        compShapes<R, false>(P, ns, sh, acos(ok ? c : R(0)), phi,
+        compShapes<R, false>(P, u, sh, acos(ok ? c : R(0)), phi,
                              (R*)nullptr);
         R rjk = R(0);
         if (NARROW)
@@ -1064,8 +1113,11 @@ __device__ __forceinline__ void compactValues(SFParams const& P,
             if (a < nr)
             {
                 PairRun const& r = runs[a];
-                R const* tab = w.W.rad + 2 * r.slot * cs;
+                R const* tab = w.W.rad + r.slot * cs;
                 R v = tab[tt] * tab[kk];
+                // Neighbors come by distance: windows that end early are
+                // zero for most whole batches.
+                if (!__any_sync(kFull, v != R(0))) continue;
                 if (NARROW)
                 {
                     R f, d;
@@ -1165,8 +1217,10 @@ pairValueKernel(__grid_constant__ SFParams const P,
         w.W.cs = cnt + 1;
         w.cells = tb.c + T.cellBeg[ec];
         for (int k = tm.tid; k < WPA * maxSF; k += Tm::kThreads) Gp[k] = R(0);
-        stageAtom<R, CT, WPA, false>(P, T, L, h, tm, pos, dist, (R*)nullptr,
-                                     (R const*)nullptr, tb.q, w.W);
+        stageAtom<R, CT, WPA, false>(
+            P, T, L, h, tm, pos, dist, (R*)nullptr, (R const*)nullptr, tb.q,
+            (unsigned short*)nullptr,
+            reinterpret_cast<unsigned*>(mine + L.oSort), w.W);
         Tm::sync();
         // Validity mask, upper triangle: (32 rows, word) per warp.
         if (T.narrow[ec])
@@ -1640,7 +1694,7 @@ __device__ __forceinline__ void compactForces(SFParams const& P,
 {
     using P2 = typename V2<R>::T;
     constexpr int S = kPairCompShapes;
-    int const ns = u.ns, nr = u.nr, cs = W.cs, none = cs - 1;
+    int const nr = u.nr, cs = W.cs, none = cs - 1;
     PairRun const* const runs = tb.r + u.run;
     PairShape const* const sh = tb.s + u.shape;
     P2 const* const C2 = reinterpret_cast<P2 const*>(C);
@@ -1657,7 +1711,7 @@ __device__ __forceinline__ void compactForces(SFParams const& P,
         c = ok ? c : R(0);
         R const dacos = -mrsqrt(R(1) - c * c);
         R phi[S], psi[S];
-        compShapes<R, true>(P, ns, sh, acos(c), phi, psi);
+        compShapes<R, true>(P, u, sh, acos(c), phi, psi);
         R rjk = R(0), ir3 = R(0);
         if (NARROW)
         {
@@ -1673,6 +1727,12 @@ __device__ __forceinline__ void compactForces(SFParams const& P,
             PairRun const& w = runs[a];
             R const* tab = W.rad + 2 * w.slot * cs;
             R const rk = tab[k];
+            R const rj = tab[p.t], drj = tab[cs + p.t];
+            // Neighbors come by distance: windows that end early are zero
+            // for most whole steps.
+            if (!__any_sync(kFull, rk != R(0)
+                                       && (rj != R(0) || drj != R(0))))
+                continue;
             R b = R(0), h = R(0);
 #pragma unroll
             for (int j = 0; j < S / 2; ++j)
@@ -1683,7 +1743,6 @@ __device__ __forceinline__ void compactForces(SFParams const& P,
                 h += cc.x * psi[2 * j];
                 h += cc.y * psi[2 * j + 1];
             }
-            R const rj = tab[p.t], drj = tab[cs + p.t];
             if (NARROW)
             {
                 R f, d;
@@ -1776,6 +1835,8 @@ pairTermKernel(__grid_constant__ SFParams const P,
     stageExpTable<R>(sm, L);
     UnitTables const tb = stageTables(T, L, sm);
     double* const F = reinterpret_cast<double*>(mine + L.oF);
+    unsigned short* const orig =
+        reinterpret_cast<unsigned short*>(mine + L.oOrig);
     Head& h = heads[tm.team];
     __syncthreads();
     for (int i = blockIdx.x * Tm::kTeams + tm.team; i < L.n;
@@ -1810,8 +1871,9 @@ pairTermKernel(__grid_constant__ SFParams const P,
             }
         }
         Tm::sync();
-        stageAtom<R, CT, WPA, true>(P, T, L, h, tm, pos, (R*)nullptr, arad, C,
-                                    tb.q, W);
+        stageAtom<R, CT, WPA, true>(
+            P, T, L, h, tm, pos, (R*)nullptr, arad, C, tb.q, orig,
+            reinterpret_cast<unsigned*>(mine + L.oSort), W);
         Tm::sync();
         // Validity masks (narrow units): (32 rows, word) blocks on and above
         // the diagonal, those below are their transposes.
@@ -2012,8 +2074,9 @@ pairTermKernel(__grid_constant__ SFParams const P,
                 double const v = sl == 0 ? Vx : (sl == 1 ? Vy : Vz);
                 double const* const a = sl == 0 ? L.dx
                                       : (sl == 1 ? L.dy : L.dz);
-                double const f = Al * a[beg + t] + v;
-                L.pairF[(beg + t) * 3 + sl] = f;
+                long const e = beg + (T.sorted[ec] ? (int)orig[t] : t);
+                double const f = Al * a[e] + v;
+                L.pairF[e * 3 + sl] = f;
                 if (WPA == 1) sx += f;
                 else F[3 * t + sl] = f;
             }

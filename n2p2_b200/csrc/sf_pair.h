@@ -53,7 +53,8 @@ struct PairUnit
     int      hasRs;       // some run has rs != 0
     int      exactMask;   // rc is the element's largest narrow cutoff
     unsigned mask;        // PK_POW2
-    int      pad;
+    int      core;        // PK_COMPACT: the shapes' common core function
+                          // (CompactCore), 0 if they differ
     unsigned prog[4];     // ladder: steps to zeta z: count in bits 0-7, then
                           // one bit per step (0: P = P^2, 1: P = P p)
     double   rc2;         // squared cutoff radius (compact: largest rc)
@@ -117,6 +118,8 @@ struct PairParams
     int runBeg[kMaxElem + 1];
     int shapeBeg[kMaxElem + 1];
     int narrow[kMaxElem];         // element has narrow units
+    int sorted[kMaxElem];         // neighbors staged by distance (the element
+                                  // has compact units)
     double narrowRc2[kMaxElem];   // largest squared cutoff of those
     int maxCells, maxFc, maxRad, numElements;
     int anyWeighted;              // some member weights by atomic number
@@ -163,7 +166,7 @@ struct PairLaunch
     // ... and into a team's region.
     int            oPos = 0, oDist = 0, oRec = 0, oFc = 0, oDfc = 0, oRad = 0,
                    oCoef = 0, oBits = 0, oPre = 0, oOrder = 0, oKey = 0,
-                   oList = 0, oPairs = 0, oRed = 0, oG = 0, oAr = 0, oF = 0;
+                   oList = 0, oOrig = 0, oSort = 0, oPairs = 0, oRed = 0, oG = 0, oAr = 0, oF = 0;
     int            tables = 0;        // bit 0: units, runs, shapes in smem,
                                       // bit 1: radial members, cells
     int            wpa = 1;           // warps per atom: 1 or 4

@@ -318,6 +318,8 @@ bool addGroup(SFParams const& P, PairTables& t, int fcBeg, int radBeg, int gi,
                     h.useInt = m.useIntPow;
                 }
                 t.shapes.push_back(h);
+                if (compact)
+                    u.core = s == 0 || u.core == h.zi ? h.zi : 0;
             }
             cells += u.nr * maxS;
             t.p.kinds |= 1 << u.kind;
@@ -365,6 +367,7 @@ void buildPairTables(SFParams const& P, PairTables& t)
             if (isRadial(P.groups[g].type)) continue;
             if (!addGroup(P, t, fcBeg, radBeg, g, p.slots, cells)) return;
             int const type = P.groups[g].type;
+            if (type >= 20) p.sorted[e] = 1;
             if (type == 3 || type == 13 || type == 21 || type == 24)
             {
                 p.narrow[e] = 1;
