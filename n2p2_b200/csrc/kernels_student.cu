@@ -62,7 +62,13 @@ __global__ void residualKernel(StudentLaunch const L)
     atomicAdd(&L.loss[1], r2);
 }
 
-// Warp per atom j: u_j over its symmetry functions.
+// Warp per atom j: u_j over its symmetry functions, lanes over the entries.
+// Bound by reading dG/dr once: the entries' residual differences are gathered
+// once per block of 32 kAdjEntries entries and stay in registers, then the
+// rows of kAdjSlots slots are read together (6,144 atoms, 437 MB: 0.297 ms
+// with the gather inside the slot loop and one slot at a time).
+constexpr int kAdjEntries = 4, kAdjSlots = 2;
+
 template <typename T>
 __global__ void __launch_bounds__(128)
 adjointKernel(StudentLaunch const L)
@@ -96,30 +102,57 @@ adjointKernel(StudentLaunch const L)
             int const ns = L.numSlots[ej][en];
             int16_t const* tab = L.slotSF + ((long)ej * kMaxElem + en)
                                             * L.maxSlots;
-            for (int sl = 0; sl < ns; ++sl)
+            for (int t0 = sb; t0 < se; t0 += 32 * kAdjEntries)
             {
-                float v = 0.0f;
-                for (int t = sb + lane; t < se; t += 32)
+                float qx[kAdjEntries], qy[kAdjEntries], qz[kAdjEntries];
+#pragma unroll
+                for (int k = 0; k < kAdjEntries; ++k)
                 {
+                    int const t = t0 + 32 * k + lane;
+                    qx[k] = qy[k] = qz[k] = 0.0f;
+                    if (t >= se) continue;
                     int const i = L.nbrIdx[b + t];
                     // A periodic self image carries no pair force, only its
                     // share of j's self derivative.
-                    float qx = -rx, qy = -ry, qz = -rz;
+                    qx[k] = -rx;
+                    qy[k] = -ry;
+                    qz[k] = -rz;
                     if (i != j)
                     {
-                        qx += L.rF[(long)i * 3 + 0];
-                        qy += L.rF[(long)i * 3 + 1];
-                        qz += L.rF[(long)i * 3 + 2];
+                        qx[k] += L.rF[(long)i * 3 + 0];
+                        qy[k] += L.rF[(long)i * 3 + 1];
+                        qz[k] += L.rF[(long)i * 3 + 2];
                     }
-                    v += qx * (float)gd[((long)sl * 3 + 0) * cnt + t]
-                       + qy * (float)gd[((long)sl * 3 + 1) * cnt + t]
-                       + qz * (float)gd[((long)sl * 3 + 2) * cnt + t];
                 }
-                v = warpSumF(v);
-                if (lane == 0) acc[tab[sl]] += v;
+                for (int sl = 0; sl < ns; sl += kAdjSlots)
+                {
+                    float v[kAdjSlots];
+#pragma unroll
+                    for (int c = 0; c < kAdjSlots; ++c)
+                    {
+                        v[c] = 0.0f;
+                        if (sl + c >= ns) continue;
+                        T const* row = gd + (long)(sl + c) * 3 * cnt + t0
+                                     + lane;
+#pragma unroll
+                        for (int k = 0; k < kAdjEntries; ++k)
+                            if (t0 + 32 * k + lane < se)
+                                v[c] += qx[k] * (float)row[32 * k]
+                                      + qy[k] * (float)row[cnt + 32 * k]
+                                      + qz[k] * (float)row[2 * cnt + 32 * k];
+                    }
+#pragma unroll
+                    for (int c = 0; c < kAdjSlots; ++c)
+                    {
+                        if (sl + c >= ns) break;
+                        v[c] = warpSumF(v[c]);
+                        if (lane == 0) acc[tab[sl + c]] += v[c];
+                    }
+                }
                 __syncwarp();
             }
         }
+        __syncwarp();
         for (int s = lane; s < nsf; s += 32)
             L.u[(long)j * L.maxSF + s] = scale * acc[s];
         __syncwarp();
