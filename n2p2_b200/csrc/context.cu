@@ -1777,6 +1777,8 @@ struct n2p2b_context
         L.maxSF = maxSF;
         L.precision = PREC_MIXED;
         L.elem = elem.as<int>();
+        L.atomsByElem = atomsByElem.as<int>();
+        L.es = es;
         L.weights = stu.w.p;
         L.G = G.p;
         L.energy = Ei.as<double>();
@@ -2094,6 +2096,8 @@ struct n2p2b_context
         L.derivatives = deriv ? 1 : 0;
         L.maxSF = maxSF;
         L.elem = elem.as<int>();
+        L.atomsByElem = atomsByElem.as<int>();
+        L.es = es;
         L.weights = nnW.as<double>();
         L.G = G.as<double>();
         L.energy = Ei.as<double>();

@@ -233,6 +233,149 @@ nnKernel(__grid_constant__ NNParams const P, NNLaunch const L)
     }
 }
 
+// The same sweeps for kNNTile atoms of one element per warp: a weight is read
+// once for all of them (the per-atom kernel reads both copies of the weights,
+// 230 KB for 92-64-64-64-1, from L2 for every atom).  Values are laid out
+// [neuron][atom], so that a lane reads the atoms' inputs as 16-byte words;
+// each sum runs over the inputs in the same order as above.  For many atoms
+// only: a warp's chain of layers takes as long as the per-atom kernel's.
+constexpr int kNNTile = 4;
+
+struct NNTileLaunch
+{
+    NNLaunch   L;
+    int const* atomsByElem;
+    ElemStarts es;
+    int        warpBeg[kMaxElem + 1];   // first warp of an element
+    int        stride;                  // values per warp
+};
+
+template <typename T>
+__global__ void __launch_bounds__(32 * kNNWarps)
+nnTileKernel(__grid_constant__ NNParams const P,
+             __grid_constant__ NNTileLaunch const N)
+{
+    extern __shared__ __align__(16) double smemD[];
+    constexpr int A = kNNTile;
+    NNLaunch const& L = N.L;
+    T const* const weights = static_cast<T const*>(L.weights);
+    T const* const Gin = static_cast<T const*>(L.G);
+    T* const dEdGout = static_cast<T*>(L.dEdG);
+    int const lane = threadIdx.x & 31;
+    int const w = threadIdx.x >> 5;
+    if (L.status[ST_FLAGS] & FLAG_ABORT) return;
+    int const wi = blockIdx.x * kNNWarps + w;
+    if (wi >= N.warpBeg[P.numElements]) return;
+    int e = 0;
+    while (wi >= N.warpBeg[e + 1]) ++e;
+    int const first = N.es.start[e] + (wi - N.warpBeg[e]) * A;
+    int const rows = min(A, N.es.start[e + 1] - first);
+    int atom[A];
+#pragma unroll
+    for (int m = 0; m < A; ++m)
+        atom[m] = N.atomsByElem[first + min(m, rows - 1)];
+    int const W = P.maxWidth;
+    T* x = reinterpret_cast<T*>(smemD) + (long)w * N.stride;  // [W][A]
+    T* y = x + W * A;
+    T* dfs = y + W * A;            // per layer [width][A], one after another
+    int const nl = P.numLayers[e];
+    int const nin = P.width[e][0];
+    for (int k = lane; k < nin; k += 32)
+#pragma unroll
+        for (int m = 0; m < A; ++m)
+            x[k * A + m] = Gin[(long)atom[m] * L.maxSF + k];
+    __syncwarp();
+    T* df = dfs;
+    for (int l = 1; l < nl; ++l)
+    {
+        int const ni = P.width[e][l - 1];
+        int const no = P.width[e][l];
+        T const* Wt = weights + P.wtoff[e][l];
+        T const* b = weights + P.boff[e][l];
+        int const act = P.act[e][l];
+        for (int o = lane; o < no; o += 32)
+        {
+            T acc[A];
+#pragma unroll
+            for (int m = 0; m < A; ++m) acc[m] = T(0);
+#pragma unroll 4
+            for (int j = 0; j < ni; ++j)
+            {
+                T const wt = Wt[(long)j * no + o];
+#pragma unroll
+                for (int m = 0; m < A; ++m) acc[m] += wt * x[j * A + m];
+            }
+#pragma unroll
+            for (int m = 0; m < A; ++m)
+            {
+                T z = acc[m] + b[o];
+                if (P.normalizeNeurons) z /= ni;
+                T v, dv;
+                activate(act, z, v, dv);
+                y[o * A + m] = v;
+                df[o * A + m] = dv;
+            }
+        }
+        __syncwarp();
+        T* const t = x;
+        x = y;
+        y = t;
+        df += no * A;
+    }
+#pragma unroll
+    for (int m = 0; m < A; ++m)
+        if (lane == 0 && m < rows) L.energy[atom[m]] = (double)x[m];
+    if (!L.derivatives) return;
+    int const nlast = P.width[e][nl - 2];
+    df -= A;                       // the output neuron's
+    T* d = y;
+    if (lane < A)
+    {
+        T v = df[lane];
+        if (P.normalizeNeurons) v /= nlast;
+        d[lane] = v;
+    }
+    __syncwarp();
+    for (int l = nl - 1; l >= 1; --l)
+    {
+        int const ni = P.width[e][l - 1];
+        int const no = P.width[e][l];
+        T const* Wm = weights + P.woff[e][l];
+        if (l > 1) df -= ni * A;
+        for (int j = lane; j < ni; j += 32)
+        {
+            T acc[A];
+#pragma unroll
+            for (int m = 0; m < A; ++m) acc[m] = T(0);
+#pragma unroll 4
+            for (int o = 0; o < no; ++o)
+            {
+                T const wm = Wm[(long)o * ni + j];
+#pragma unroll
+                for (int m = 0; m < A; ++m) acc[m] += wm * d[o * A + m];
+            }
+#pragma unroll
+            for (int m = 0; m < A; ++m)
+            {
+                if (l > 1)
+                {
+                    acc[m] *= df[j * A + m];
+                    if (P.normalizeNeurons) acc[m] /= P.width[e][l - 2];
+                }
+                x[j * A + m] = acc[m];
+            }
+        }
+        __syncwarp();
+        T* const t = x;
+        x = d;
+        d = t;
+    }
+    for (int k = lane; k < nin; k += 32)
+#pragma unroll
+        for (int m = 0; m < A; ++m)
+            if (m < rows) dEdGout[(long)atom[m] * L.maxSF + k] = d[k * A + m];
+}
+
 // Pass 1: warp per owner atom j.  T is the type of dE/dG and dG/dr (double,
 // or float in the mixed form); products and sums are formed in FP64.
 template <typename T>
@@ -538,9 +681,57 @@ void launchEnergyBatch(BatchEnergyLaunch const& L, cudaStream_t s)
     energyBatchKernel<<<L.numStructs > 0 ? L.numStructs : 1, 256, 0, s>>>(L);
 }
 
+namespace
+{
+
+template <typename T>
+void launchNNTile(NNParams const& P, NNTileLaunch const& N, int blocks,
+                  std::size_t shm, cudaStream_t s)
+{
+    cudaFuncSetAttribute(nnTileKernel<T>,
+                         cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)shm);
+    nnTileKernel<T><<<blocks, 32 * kNNWarps, shm, s>>>(P, N);
+}
+
+} // namespace
+
 void launchNeuralNetworks(NNParams const& P, NNLaunch const& L,
                           cudaStream_t s)
 {
+    // Tiles once every multiprocessor has four blocks of them, and where
+    // their values fit.
+    if (L.atomsByElem && L.n >= kNNTile * kNNWarps * 4 * 148)
+    {
+        NNTileLaunch N;
+        N.L = L;
+        N.atomsByElem = L.atomsByElem;
+        N.es = L.es;
+        int most = 0;
+        N.warpBeg[0] = 0;
+        for (int e = 0; e < kMaxElem; ++e)
+        {
+            int const c = e < P.numElements
+                ? L.es.start[e + 1] - L.es.start[e] : 0;
+            N.warpBeg[e + 1] = N.warpBeg[e] + (c + kNNTile - 1) / kNNTile;
+            int v = 0;
+            for (int l = 1; e < P.numElements && l < P.numLayers[e]; ++l)
+                v += P.width[e][l];
+            most = v > most ? v : most;
+        }
+        N.stride = (2 * P.maxWidth + most) * kNNTile;
+        bool const f32 = L.precision != PREC_FP64;
+        std::size_t const shm = (f32 ? sizeof(float) : sizeof(double))
+                              * (std::size_t)kNNWarps * N.stride;
+        if (shm <= 56 * 1024)
+        {
+            int const blocks = (N.warpBeg[kMaxElem] + kNNWarps - 1) / kNNWarps;
+            noteLaunches(1);
+            if (f32) launchNNTile<float>(P, N, blocks, shm, s);
+            else launchNNTile<double>(P, N, blocks, shm, s);
+            return;
+        }
+    }
     bool const f = L.precision != PREC_FP64;
     std::size_t const shm = (f ? sizeof(float) : sizeof(double))
                           * (std::size_t)kNNWarps * P.maxWidth
