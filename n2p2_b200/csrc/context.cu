@@ -1981,18 +1981,17 @@ struct n2p2b_context
         launchStudentRange(R, stream);
         if (pairUsable())
         {
-            // The values of the other route differ in rounding: the range
-            // holds for both, so that no atom of a training frame is gated
-            // whichever computes its symmetry functions later.
+            // The values of the two routes differ in rounding (the current
+            // ones are from either): the range holds for both, so that no
+            // atom of a training frame is gated whichever computes its
+            // symmetry functions later.
             Gother.ensure(realBytes() * n * maxSF);
-            if (haveDGdr)
-            {
-                PairLaunch L = pairLaunch();
-                L.G = Gother.p;
-                launchPair(0, sfp, pt.p, ptDev, L, stream);
-            }
-            else enqueueStoredSF(false, Gother.p);
             R.G = Gother.p;
+            enqueueStoredSF(false, Gother.p);
+            launchStudentRange(R, stream);
+            PairLaunch L = pairLaunch();
+            L.G = Gother.p;
+            launchPair(0, sfp, pt.p, ptDev, L, stream);
             launchStudentRange(R, stream);
         }
         checkLaunch("training range");
