@@ -376,7 +376,7 @@ struct n2p2b_context
     ElemStarts   es{};
     int          numCells = 0;
     DevBuf       posIn, pos, elem, atomsByElem;
-    DevBuf       cellOf, cellCount, cellFill, cellStart, cellAtoms, cellStatus;
+    DevBuf       cellOf, cellCount, cellStart, cellPos, cellEl, cellStatus;
     DevBuf       nbrCount, nbrCountElem, nbrOff;
     long         capacity = 0;
     DevBuf       keyTmp, key, nbrIdx, nbrEl, dx, dy, dz, dd, entryAtom, mirror;
@@ -476,8 +476,8 @@ struct n2p2b_context
             b->release();
         for (DevBuf* b : {&sfScale, &nnW, &slotSF, &tcW[0], &tcF[0], &tcW[1],
                           &tcF[1], &ewRange, &ewPerAtom, &posIn, &pos, &elem,
-                          &atomsByElem, &cellOf, &cellCount, &cellFill,
-                          &cellStart, &cellAtoms, &cellStatus, &nbrCount,
+                          &atomsByElem, &cellOf, &cellCount, &cellStart,
+                          &cellPos, &cellEl, &cellStatus, &nbrCount,
                           &nbrCountElem, &nbrOff, &keyTmp, &key, &nbrIdx,
                           &nbrEl, &dx, &dy, &dz, &dd, &entryAtom, &mirror,
                           &pairF, &dGdr, &G, &Gother, &dEdG, &dGdrSelf, &Ei,
@@ -1190,9 +1190,9 @@ struct n2p2b_context
     {
         int const ne = pot.numElements();
         cellOf.ensure(sizeof(int) * n);
-        cellAtoms.ensure(sizeof(int) * n);
+        cellPos.ensure(sizeof(float4) * n);
+        cellEl.ensure(n);
         cellCount.ensure(sizeof(int) * (numCells + 1));
-        cellFill.ensure(sizeof(int) * (numCells + 1));
         cellStart.ensure(sizeof(int) * (numCells + 1));
         cellStatus.ensure(sizeof(int) * ST_NUM);
         nbrCount.ensure(sizeof(int) * n);
@@ -1309,9 +1309,15 @@ struct n2p2b_context
         if (externalNL) return;      // the caller's list is already in place
         // Small single structures run as a batch of one: every pair of atoms
         // is a candidate, but there are no cells to build and the entries
-        // come in key order (nothing to sort).  192 atoms 0.206 -> 0.044 ms,
-        // 1,080 atoms 0.148 -> 0.110 ms, 1,728 atoms 0.111 -> 0.130 ms.
-        bool const small = numStructs == 0 && n <= 1536 && nlp.nimg <= 128;
+        // come in key order (nothing to sort).  Against the cells, water:
+        // 192 atoms 0.045 / 0.103 ms, 600 0.076 / 0.081, 768 0.085 / 0.071,
+        // 1,536 0.139 / 0.084.  Open structures against every pair in FP64:
+        // 300 atoms 0.055 / 0.062, 1,536 0.137 / 0.118.  Periodic boxes
+        // that cannot be cut into cells (skewed or thin) leave only a
+        // search of all their images: 1,536 atoms 0.083 / 0.169.
+        bool const uncut = nlp.ncell[0] == 0 && nlp.nimg > 1;
+        bool const small = numStructs == 0 && nlp.nimg <= 128
+                        && (uncut || n <= 640);
         if (numStructs > 0 || small)
         {
             NLBatchLaunch B;
@@ -1375,8 +1381,8 @@ struct n2p2b_context
         L.cellOf = cellOf.as<int>();
         L.cellCount = cellCount.as<int>();
         L.cellStart = cellStart.as<int>();
-        L.cellFill = cellFill.as<int>();
-        L.cellAtoms = cellAtoms.as<int>();
+        L.cellPos = cellPos.as<float4>();
+        L.cellEl = cellEl.as<int8_t>();
         L.cellScanStatus = cellStatus.as<int>();
         L.nbrCount = nbrCount.as<int>();
         L.nbrCountElem = nbrCountElem.as<int>();

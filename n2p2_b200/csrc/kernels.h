@@ -36,8 +36,8 @@ struct NLLaunch
     int*                cellOf = nullptr;
     int*                cellCount = nullptr;
     int*                cellStart = nullptr;
-    int*                cellFill = nullptr;
-    int*                cellAtoms = nullptr;
+    float4*             cellPos = nullptr; // by cell: FP32 position, atom
+    int8_t*             cellEl = nullptr;  // by cell: element
     int*                cellScanStatus = nullptr;
     int*                nbrCount = nullptr;
     int*                nbrCountElem = nullptr;

@@ -20,7 +20,8 @@
 //    with periodic wrap.  Used when every box vector's perpendicular width
 //    exceeds rc (then pbc = 1) and every atom lies inside the cell (fractional
 //    coordinates in [0, 1], true after remap): all neighbors then have
-//    |bc| <= 1 and sit in adjacent cells.  Hits are ranked by key per atom.
+//    |bc| <= 1 and sit in adjacent cells.  An FP32 distance decides away from
+//    the cutoff.  Hits are ranked by key per atom.
 //  * brute path: all (j, bc) candidates in key order, the reference's own
 //    enumeration; used for small or skewed cells, atoms outside the cell and
 //    non-periodic structures.
@@ -110,16 +111,23 @@ __global__ void nlPrepareKernel(int n, double const* __restrict__ posIn,
     }
 }
 
-__global__ void nlBinKernel(int n, int const* __restrict__ cellOf,
+// Atoms by cell, with FP32 positions for the distance test (one 16-byte load
+// per candidate).  Counts the cells down: cellCount is zero afterwards.
+__global__ void nlBinKernel(int n, double const* __restrict__ pos,
+                            int const* __restrict__ elem,
+                            int const* __restrict__ cellOf,
                             int const* __restrict__ cellStart,
-                            int* __restrict__ cellFill,
-                            int* __restrict__ cellAtoms)
+                            int* __restrict__ cellCount,
+                            float4* __restrict__ cellPos,
+                            int8_t* __restrict__ cellEl)
 {
     int const i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     int const c = cellOf[i];
-    int const slot = atomicAdd(&cellFill[c], 1);
-    cellAtoms[cellStart[c] + slot] = i;
+    int const at = cellStart[c] + atomicSub(&cellCount[c], 1) - 1;
+    cellPos[at] = make_float4((float)pos[3 * i], (float)pos[3 * i + 1],
+                              (float)pos[3 * i + 2], __int_as_float(i));
+    cellEl[at] = (int8_t)elem[i];
 }
 
 // Exact reference displacement and cutoff test for candidate (j, bc).
@@ -172,149 +180,288 @@ __device__ __forceinline__ unsigned long long nlKey(int ej, int j, int img,
            + (unsigned long long)img;
 }
 
-// Stencil cell c + d (d in {-1,0,1}^3 from s in [0,27)) with periodic wrap;
-// returns the cell and the image bc of the atoms found there.
-__device__ __forceinline__ int stencilCell(NLParams const& p, int const c[3],
-                                           int s, int bc[3])
+// A list's entries: key order, displacements, owner.
+struct ListOut
 {
-    int const d[3] = {s / 9 - 1, (s / 3) % 3 - 1, s % 3 - 1};
-    int cc[3];
-#pragma unroll
-    for (int k = 0; k < 3; ++k)
-    {
-        int v = c[k] + d[k];
-        int w = 0;
-        if (v < 0)                 { v += p.ncell[k]; w = -1; }
-        else if (v >= p.ncell[k])  { v -= p.ncell[k]; w = 1; }
-        cc[k] = v;
-        bc[k] = -w;
-    }
-    return (cc[0] * p.ncell[1] + cc[1]) * p.ncell[2] + cc[2];
+    unsigned long long* key;
+    int*                nbrIdx;
+    int8_t*             nbrEl;
+    double*             dx;
+    double*             dy;
+    double*             dz;
+    double*             dd;
+    int*                entryAtom;
+};
+
+__device__ __forceinline__ void writeEntry(ListOut const& o, long at, int i,
+                                           unsigned long long key, int j,
+                                           int ej, double const dr[3])
+{
+    double const n2 = __dadd_rn(__dadd_rn(__dmul_rn(dr[0], dr[0]),
+                                          __dmul_rn(dr[1], dr[1])),
+                                __dmul_rn(dr[2], dr[2]));
+    o.key[at] = key;
+    o.nbrIdx[at] = j;
+    o.nbrEl[at] = (int8_t)ej;
+    o.dx[at] = dr[0];
+    o.dy[at] = dr[1];
+    o.dz[at] = dr[2];
+    o.dd[at] = __dsqrt_rn(n2);
+    o.entryAtom[at] = i;
 }
 
 // ---------------------------------------------------------------------------
 // Cell path.  Warp per atom.  MODE 0 counts hits (total and per element);
-// MODE 1 writes the hits' keys, unsorted, into keyTmp[nbrOff[i] ...].
+// MODE 1 collects the hits' keys, ranks them and writes the entries.
+//
+// Bound by the distance tests (6 to 7 candidates per neighbor).  The cells of
+// one (c0, c1) row lie one after another in memory, so the 27 cells are 9
+// runs of three cells (and the wrapped ends): a lane holds a run, the warp
+// walks it 32 candidates at a time.  An FP32 distance decides outside
+// rc^2 -+ slack: coordinates inside the cell are at most B = sum_k |a_k|, an
+// image shift as well, so a component of the difference errs by less than
+// 32 B 2^-24 and r^2 near the cutoff by 6 rc err + 3 err^2 (slack: four
+// times that, at least 1e-4 rc^2); between them nlTest does.  Up to
+// kCellHits keys of 32 bits are ranked in shared memory (one pass of 16-byte
+// reads for four keys a lane), others in keyTmp.  24,576 water atoms, both
+// modes, ranks and entries: 0.37 ms with an FP64 test of every candidate and
+// 64-bit keys ranked in global memory, 0.20 ms so.
 // ---------------------------------------------------------------------------
+constexpr int kCellHits = 256, kCellWarps = 4;
+
 template <int MODE>
-__global__ void nlCellKernel(int n, NLParams p, int numElements,
-                             double const* __restrict__ pos,
-                             int const* __restrict__ elem,
-                             int const* __restrict__ cellOf,
-                             int const* __restrict__ cellStart,
-                             int const* __restrict__ cellCount,
-                             int const* __restrict__ cellAtoms,
-                             int* __restrict__ nbrCount,
-                             int* __restrict__ nbrCountElem,
-                             int const* __restrict__ nbrOff,
-                             unsigned long long* __restrict__ keyTmp,
-                             int const* __restrict__ status)
+__global__ void __launch_bounds__(32 * kCellWarps)
+nlCellKernel(int n, __grid_constant__ NLParams const p, int numElements,
+             double const* __restrict__ pos, int const* __restrict__ elem,
+             int const* __restrict__ cellOf,
+             int const* __restrict__ cellStart,
+             float4 const* __restrict__ cellPos,
+             int8_t const* __restrict__ cellEl, int* __restrict__ nbrCount,
+             int* __restrict__ nbrCountElem, int const* __restrict__ nbrOff,
+             unsigned long long* __restrict__ keyTmp, ListOut const out,
+             int const* __restrict__ status)
 {
+    __shared__ __align__(16) unsigned found[MODE == 1 ? kCellWarps : 1]
+                                           [MODE == 1 ? kCellHits : 4];
+    __shared__ unsigned order[MODE == 1 ? kCellWarps : 1]
+                             [MODE == 1 ? kCellHits : 1];
     if (status[ST_FLAGS] & (FLAG_OUTSIDE_CELL | FLAG_ABORT)) return;
     int const lane = threadIdx.x & 31;
-    int const i = (int)((blockIdx.x * (long)blockDim.x + threadIdx.x) >> 5);
+    int const warp = threadIdx.x >> 5;
+    int const i = blockIdx.x * kCellWarps + warp;
     if (i >= n) return;
     double const ri[3] = {pos[3 * i], pos[3 * i + 1], pos[3 * i + 2]};
-    int const cell = cellOf[i];
-    int c[3];
-    c[2] = cell % p.ncell[2];
-    c[1] = (cell / p.ncell[2]) % p.ncell[1];
-    c[0] = cell / (p.ncell[2] * p.ncell[1]);
-    int cntElem[kMaxElem];
-#pragma unroll
-    for (int e = 0; e < kMaxElem; ++e) cntElem[e] = 0;
-    int total = 0;
-    long const base = (MODE == 1) ? (long)nbrOff[i] : 0;
-    // Lane s < 27 holds stencil cell s (first atom, count, image); the
-    // candidates of all 27 cells form one list of `nc` entries that the
-    // warp walks 32 at a time, so lanes stay busy across cell boundaries.
-    int cs = 0, cn = 0, bcw = 0;
+    long const base = MODE == 1 ? (long)nbrOff[i] : 0;
+    int const cnt = MODE == 1 ? nbrOff[i + 1] - (int)base : 0;
+    bool const small = cnt <= kCellHits
+        && (unsigned long long)numElements * n * p.nimg < 0xffffffffull;
+    // Lane 3 r + k < 27: row r of the stencil; k = 0 its cells inside the
+    // box, k = 1 and 2 the ones wrapped below and above.
+    int first = 0, len = 0, img = 0;
+    float sx = 0.0f, sy = 0.0f, sz = 0.0f;
     if (lane < 27)
     {
-        int bc[3];
-        int const cc = stencilCell(p, c, lane, bc);
-        cs = cellStart[cc];
-        cn = cellCount[cc];
-        bcw = (bc[0] + 1) * 9 + (bc[1] + 1) * 3 + (bc[2] + 1);
-    }
-    int incl = cn;
+        int const cell = cellOf[i];
+        int const c2 = cell % p.ncell[2];
+        int v[2] = {cell / (p.ncell[2] * p.ncell[1]) + lane / 9 - 1,
+                    (cell / p.ncell[2]) % p.ncell[1] + (lane / 3) % 3 - 1};
+        int bc[3] = {0, 0, 0};
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1)
-    {
-        int const v = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += v;
+        for (int k = 0; k < 2; ++k)
+        {
+            if (v[k] < 0) { v[k] += p.ncell[k]; bc[k] = 1; }
+            else if (v[k] >= p.ncell[k]) { v[k] -= p.ncell[k]; bc[k] = -1; }
+        }
+        int const row = (v[0] * p.ncell[1] + v[1]) * p.ncell[2];
+        int lo = max(c2 - 1, 0), hi = min(c2 + 1, p.ncell[2] - 1);
+        if (lane % 3 == 1)
+        {
+            bc[2] = 1;
+            lo = p.ncell[2] - 1;
+            hi = c2 == 0 ? lo : lo - 1;
+        }
+        if (lane % 3 == 2)
+        {
+            bc[2] = -1;
+            lo = 0;
+            hi = c2 == p.ncell[2] - 1 ? 0 : -1;
+        }
+        if (lo <= hi)
+        {
+            first = cellStart[row + lo];
+            len = cellStart[row + hi + 1] - first;
+        }
+        img = imgIndex(p, bc[0], bc[1], bc[2]);
+        float const b0 = (float)bc[0], b1 = (float)bc[1], b2 = (float)bc[2];
+        sx = b0 * (float)p.box[0][0] + b1 * (float)p.box[1][0]
+           + b2 * (float)p.box[2][0];
+        sy = b0 * (float)p.box[0][1] + b1 * (float)p.box[1][1]
+           + b2 * (float)p.box[2][1];
+        sz = b0 * (float)p.box[0][2] + b1 * (float)p.box[1][2]
+           + b2 * (float)p.box[2][2];
     }
-    int const nc = __shfl_sync(0xffffffffu, incl, 31);
-    for (int q0 = 0; q0 < nc; q0 += 32)
-    {
-        int const q = q0 + lane;
-        // Cell of candidate q: the number of cells whose inclusive count
-        // end is <= q (ends are nondecreasing over lanes).
-        int sc = 0;
+    float const x = (float)ri[0], y = (float)ri[1], z = (float)ri[2];
+    float const rc2 = (float)p.rc2;
+    float B = 0.0f;
 #pragma unroll
-        for (int step = 16; step >= 1; step >>= 1)
+    for (int c = 0; c < 3; ++c)
+        B = fmaxf(B, fabsf((float)p.box[0][c]) + fabsf((float)p.box[1][c])
+                     + fabsf((float)p.box[2][c]));
+    float const err = 32.0f * B * 5.9604645e-8f;
+    float const slack = fmaxf(1e-4f * rc2, 4.0f * (6.0f * sqrtf(rc2) * err
+                                                   + 3.0f * err * err));
+    float const above = rc2 + slack, below = rc2 - slack;
+    int const home = imgIndex(p, 0, 0, 0);
+    // Hits per element: 16 bits each.
+    unsigned long long cntElem[(kMaxElem + 3) / 4] = {};
+    int total = 0;
+    unsigned runs = __ballot_sync(0xffffffffu, len > 0);
+    while (runs)
+    {
+        int const src = __ffs(runs) - 1;
+        runs &= runs - 1;
+        int const f = __shfl_sync(0xffffffffu, first, src);
+        int const m = __shfl_sync(0xffffffffu, len, src);
+        int const im = __shfl_sync(0xffffffffu, img, src);
+        float const x0 = x + __shfl_sync(0xffffffffu, sx, src);
+        float const y0 = y + __shfl_sync(0xffffffffu, sy, src);
+        float const z0 = z + __shfl_sync(0xffffffffu, sz, src);
+#pragma unroll 4
+        for (int q = lane; q < ((m + 31) & ~31); q += 32)
         {
-            int const probe = sc + step - 1;
-            int const v = __shfl_sync(0xffffffffu, incl, probe < 27 ? probe
-                                                                    : 26);
-            if (probe < 27 && v <= q) sc += step;
-        }
-        int const src = sc < 27 ? sc : 26;
-        int const endS = __shfl_sync(0xffffffffu, incl, src);
-        int const cnS = __shfl_sync(0xffffffffu, cn, src);
-        int const csS = __shfl_sync(0xffffffffu, cs, src);
-        int const bcS = __shfl_sync(0xffffffffu, bcw, src);
-        bool hit = false;
-        int j = 0;
-        int bc[3] = {bcS / 9 - 1, (bcS / 3) % 3 - 1, bcS % 3 - 1};
-        int const img = imgIndex(p, bc[0], bc[1], bc[2]);
-        if (q < nc)
-        {
-            j = cellAtoms[csS + (q - (endS - cnS))];
-            bool const zeroShift = (bc[0] == 0 && bc[1] == 0 && bc[2] == 0);
-            if (!(j == i && zeroShift))
+            bool hit = false;
+            int j = 0;
+            if (q < m)
             {
-                double dr[3];
-                hit = nlTest(p, ri, pos, j, bc[0], bc[1], bc[2], dr);
-            }
-        }
-        {
-            unsigned const m = __ballot_sync(0xffffffffu, hit);
-            if (MODE == 0)
-            {
-                if (hit)
+                float4 const a = cellPos[f + q];
+                j = __float_as_int(a.w);
+                float const dx = x0 - a.x, dy = y0 - a.y, dz = z0 - a.z;
+                float const r2 = dx * dx + dy * dy + dz * dz;
+                hit = r2 <= above && !(j == i && im == home);
+                if (hit && r2 >= below)
                 {
-                    int const ej = elem[j];
-#pragma unroll
-                    for (int e = 0; e < kMaxElem; ++e) cntElem[e] += (ej == e);
+                    int b0, b1, b2;
+                    double dr[3];
+                    imgDecode(p, im, b0, b1, b2);
+                    hit = nlTest(p, ri, pos, j, b0, b1, b2, dr);
                 }
             }
-            else if (hit)
+            unsigned const hits = __ballot_sync(0xffffffffu, hit);
+            if (hit)
             {
-                int const off = total + __popc(m & ((1u << lane) - 1u));
-                keyTmp[base + off] = nlKey(elem[j], j, img, n, p.nimg);
+                int const ej = cellEl[f + q];
+                if (MODE == 0)
+                {
+#pragma unroll
+                    for (int k = 0; k < (kMaxElem + 3) / 4; ++k)
+                        if (ej >> 2 == k)
+                            cntElem[k] += 1ull << (16 * (ej & 3));
+                }
+                else
+                {
+                    int const at = total
+                                 + __popc(hits & ((1u << lane) - 1u));
+                    unsigned long long const key =
+                        nlKey(ej, j, im, n, p.nimg);
+                    if (at < cnt)
+                    {
+                        if (small) found[warp][at] = (unsigned)key;
+                        else keyTmp[base + at] = key;
+                    }
+                }
             }
-            total += __popc(m);
+            total += __popc(hits);
         }
     }
     if (MODE == 0)
     {
         for (int e = 0; e < numElements; ++e)
         {
-            int v = cntElem[e];
+            unsigned long long w = 0;
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1)
-                v += __shfl_xor_sync(0xffffffffu, v, o);
+            for (int k = 0; k < (kMaxElem + 3) / 4; ++k)
+                if (e >> 2 == k) w = cntElem[k];
+            int const v = __reduce_add_sync(
+                0xffffffffu, (int)(w >> (16 * (e & 3))) & 0xffff);
             if (lane == 0) nbrCountElem[(long)i * numElements + e] = v;
         }
         if (lane == 0) nbrCount[i] = total;
+        return;
+    }
+    unsigned* const mine = found[warp];
+    unsigned* const sorted = order[warp];
+    if (small)
+    {
+        // Pad to a whole 16-byte word with a key above all.
+        if (lane < 4 && cnt + lane < ((cnt + 3) & ~3))
+            mine[cnt + lane] = 0xffffffffu;
+        __syncwarp();
+        for (int t0 = 0; t0 < cnt; t0 += 128)
+        {
+            unsigned k[4];
+            int r[4] = {0, 0, 0, 0};
+#pragma unroll
+            for (int c = 0; c < 4; ++c)
+            {
+                int const t = t0 + 32 * c + lane;
+                k[c] = t < cnt ? mine[t] : 0u;
+            }
+            for (int u = 0; u < cnt; u += 4)
+            {
+                uint4 const v = *reinterpret_cast<uint4 const*>(mine + u);
+#pragma unroll
+                for (int c = 0; c < 4; ++c)
+                    r[c] += (v.x < k[c]) + (v.y < k[c]) + (v.z < k[c])
+                          + (v.w < k[c]);
+            }
+#pragma unroll
+            for (int c = 0; c < 4; ++c)
+                if (t0 + 32 * c + lane < cnt) sorted[r[c]] = k[c];
+        }
+    }
+    else
+    {
+        __syncwarp();
+        for (int t = lane; t < cnt; t += 32)
+        {
+            unsigned long long const k = keyTmp[base + t];
+            int r = 0;
+            for (int u = 0; u < cnt; ++u) r += (keyTmp[base + u] < k);
+            out.key[base + r] = k;
+        }
+    }
+    __syncwarp();
+    for (int t = lane; t < cnt; t += 32)
+    {
+        unsigned long long key;
+        int j, im;
+        if (small)
+        {
+            unsigned const k = sorted[t];
+            unsigned const q = k / (unsigned)p.nimg;
+            im = (int)(k - q * (unsigned)p.nimg);
+            j = (int)(q % (unsigned)n);
+            key = k;
+        }
+        else
+        {
+            key = out.key[base + t];
+            unsigned long long const q = key / (unsigned long long)p.nimg;
+            im = (int)(key - q * (unsigned long long)p.nimg);
+            j = (int)(q % (unsigned long long)n);
+        }
+        int b0, b1, b2;
+        imgDecode(p, im, b0, b1, b2);
+        double dr[3];
+        nlTest(p, ri, pos, j, b0, b1, b2, dr);
+        writeEntry(out, base + t, i, key, j, elem[j], dr);
     }
 }
 
 // ---------------------------------------------------------------------------
 // Brute path.  Warp per atom, candidates enumerated in key order:
 // element-major, then j ascending (atomsByElem is sorted per element), then
-// image.  MODE 0 counts; MODE 1 writes keys (already sorted) into key[].
+// image.  MODE 0 counts; MODE 1 writes the entries.
 // `onlyIfOutside`: the cell path was eligible, so run only if some atom was
 // found outside the cell.
 // ---------------------------------------------------------------------------
@@ -327,7 +474,7 @@ __global__ void nlBruteKernel(int n, NLParams p, int numElements,
                               int* __restrict__ nbrCount,
                               int* __restrict__ nbrCountElem,
                               int const* __restrict__ nbrOff,
-                              unsigned long long* __restrict__ key,
+                              ListOut const out,
                               int const* __restrict__ status)
 {
     int const flags = status[ST_FLAGS];
@@ -350,6 +497,7 @@ __global__ void nlBruteKernel(int n, NLParams p, int numElements,
             long const c = c0 + lane;
             bool hit = false;
             int j = 0, img = 0;
+            double dr[3];
             if (c < ncand)
             {
                 j = atomsByElem[eb + (int)(c / nimg)];
@@ -357,16 +505,14 @@ __global__ void nlBruteKernel(int n, NLParams p, int numElements,
                 int b0, b1, b2;
                 imgDecode(p, img, b0, b1, b2);
                 if (!(j == i && b0 == 0 && b1 == 0 && b2 == 0))
-                {
-                    double dr[3];
                     hit = nlTest(p, ri, pos, j, b0, b1, b2, dr);
-                }
             }
             unsigned const m = __ballot_sync(0xffffffffu, hit);
             if (MODE == 1 && hit)
             {
                 int const off = total + __popc(m & ((1u << lane) - 1u));
-                key[base + off] = nlKey(e, j, img, n, nimg);
+                writeEntry(out, base + off, i, nlKey(e, j, img, n, nimg), j,
+                           e, dr);
             }
             total += __popc(m);
             cntE += __popc(m);
@@ -485,66 +631,6 @@ nlScanKernel(int n, int const* __restrict__ cnt, int* __restrict__ off,
     }
 }
 
-// Warp per atom: (cell path) rank the unsorted keys; then decode every entry
-// into the structure-of-arrays neighbor list with the exact displacement.
-__global__ void nlFinishKernel(int n, NLParams p, int sortKeys,
-                               double const* __restrict__ pos,
-                               int const* __restrict__ elem,
-                               int const* __restrict__ nbrOff,
-                               unsigned long long const* __restrict__ keyTmp,
-                               unsigned long long* __restrict__ key,
-                               int* __restrict__ nbrIdx,
-                               int8_t* __restrict__ nbrEl,
-                               double* __restrict__ dx,
-                               double* __restrict__ dy,
-                               double* __restrict__ dz,
-                               double* __restrict__ dd,
-                               int const* __restrict__ status)
-{
-    int const flags = status[ST_FLAGS];
-    if (flags & FLAG_ABORT) return;
-    // The cell path's keys are only valid if it ran.
-    if (sortKeys && (flags & FLAG_OUTSIDE_CELL)) sortKeys = 0;
-    int const lane = threadIdx.x & 31;
-    int const i = (int)((blockIdx.x * (long)blockDim.x + threadIdx.x) >> 5);
-    if (i >= n) return;
-    long const b = nbrOff[i];
-    int const cnt = nbrOff[i + 1] - nbrOff[i];
-    if (sortKeys)
-    {
-        for (int t = lane; t < cnt; t += 32)
-        {
-            unsigned long long const k = keyTmp[b + t];
-            int r = 0;
-            for (int u = 0; u < cnt; ++u) r += (keyTmp[b + u] < k);
-            key[b + r] = k;
-        }
-        __syncwarp();
-    }
-    double const ri[3] = {pos[3 * i], pos[3 * i + 1], pos[3 * i + 2]};
-    unsigned long long const nimg = (unsigned long long)p.nimg;
-    for (int t = lane; t < cnt; t += 32)
-    {
-        unsigned long long const k = key[b + t];
-        int const img = (int)(k % nimg);
-        unsigned long long const q = k / nimg;
-        int const j = (int)(q % (unsigned long long)n);
-        int b0, b1, b2;
-        imgDecode(p, img, b0, b1, b2);
-        double dr[3];
-        nlTest(p, ri, pos, j, b0, b1, b2, dr);
-        double const n2 = __dadd_rn(__dadd_rn(__dmul_rn(dr[0], dr[0]),
-                                              __dmul_rn(dr[1], dr[1])),
-                                    __dmul_rn(dr[2], dr[2]));
-        nbrIdx[b + t] = j;
-        nbrEl[b + t] = (int8_t)elem[j];
-        dx[b + t] = dr[0];
-        dy[b + t] = dr[1];
-        dz[b + t] = dr[2];
-        dd[b + t] = __dsqrt_rn(n2);
-    }
-}
-
 // Thread per entry: position of the mirror entry (j -> i, -bc) in j's list,
 // found by binary search over j's sorted keys.  Exists by symmetry: IEEE
 // rounding is sign-symmetric, so the mirror displacement is exactly -dr.
@@ -583,17 +669,6 @@ __global__ void nlMirrorKernel(int n, int nimg,
     }
 }
 
-// Thread per atom: owner atom of every entry (for entry-parallel kernels).
-__global__ void nlEntryAtomKernel(int n, int const* __restrict__ nbrOff,
-                                  int* __restrict__ entryAtom,
-                                  int const* __restrict__ status)
-{
-    if (status[ST_FLAGS] & FLAG_ABORT) return;
-    int const i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    for (int e = nbrOff[i]; e < nbrOff[i + 1]; ++e) entryAtom[e] = i;
-}
-
 // ---------------------------------------------------------------------------
 // Host-side launchers
 // ---------------------------------------------------------------------------
@@ -611,12 +686,12 @@ void launchNeighborList(NLLaunch const& L, cudaStream_t s)
     int const gAtoms = (n + tb - 1) / tb;
     int const warpsPerBlock = 4;
     int const gWarp = (n + warpsPerBlock - 1) / warpsPerBlock;
+    int const gCell = (n + kCellWarps - 1) / kCellWarps;
     bool const cellEligible = L.p.ncell[0] > 0;
+    ListOut const out{L.key, L.nbrIdx, L.nbrEl, L.dx, L.dy, L.dz, L.dd,
+                      L.entryAtom};
     if (cellEligible)
-    {
         cudaMemsetAsync(L.cellCount, 0, sizeof(int) * (size_t)L.numCells, s);
-        cudaMemsetAsync(L.cellFill, 0, sizeof(int) * (size_t)L.numCells, s);
-    }
     nlPrepareKernel<<<gAtoms, tb, 0, s>>>(n, L.posIn, L.doRemap, L.normalize,
                                           L.convLength, L.pb, L.p, L.pos,
                                           L.cellOf, L.cellCount, L.status);
@@ -624,36 +699,30 @@ void launchNeighborList(NLLaunch const& L, cudaStream_t s)
     {
         nlScanKernel<<<1, 1024, 0, s>>>(L.numCells, L.cellCount, L.cellStart,
                                         0x7fffffffL, L.cellScanStatus);
-        nlBinKernel<<<gAtoms, tb, 0, s>>>(n, L.cellOf, L.cellStart,
-                                          L.cellFill, L.cellAtoms);
-        nlCellKernel<0><<<gWarp, 32 * warpsPerBlock, 0, s>>>(
+        nlBinKernel<<<gAtoms, tb, 0, s>>>(n, L.pos, L.elem, L.cellOf,
+                                          L.cellStart, L.cellCount, L.cellPos,
+                                          L.cellEl);
+        nlCellKernel<0><<<gCell, 32 * kCellWarps, 0, s>>>(
             n, L.p, L.numElements, L.pos, L.elem, L.cellOf, L.cellStart,
-            L.cellCount, L.cellAtoms, L.nbrCount, L.nbrCountElem, L.nbrOff,
-            L.keyTmp, L.status);
+            L.cellPos, L.cellEl, L.nbrCount, L.nbrCountElem, L.nbrOff,
+            L.keyTmp, out, L.status);
     }
     nlBruteKernel<0><<<gWarp, 32 * warpsPerBlock, 0, s>>>(
         n, L.p, L.numElements, cellEligible ? 1 : 0, L.pos, L.atomsByElem,
-        L.es, L.nbrCount, L.nbrCountElem, L.nbrOff, L.key, L.status);
+        L.es, L.nbrCount, L.nbrCountElem, L.nbrOff, out, L.status);
     nlScanKernel<<<1, 1024, 0, s>>>(n, L.nbrCount, L.nbrOff, L.capacity,
                                     L.status);
     if (cellEligible)
-    {
-        nlCellKernel<1><<<gWarp, 32 * warpsPerBlock, 0, s>>>(
+        nlCellKernel<1><<<gCell, 32 * kCellWarps, 0, s>>>(
             n, L.p, L.numElements, L.pos, L.elem, L.cellOf, L.cellStart,
-            L.cellCount, L.cellAtoms, L.nbrCount, L.nbrCountElem, L.nbrOff,
-            L.keyTmp, L.status);
-    }
+            L.cellPos, L.cellEl, L.nbrCount, L.nbrCountElem, L.nbrOff,
+            L.keyTmp, out, L.status);
     nlBruteKernel<1><<<gWarp, 32 * warpsPerBlock, 0, s>>>(
         n, L.p, L.numElements, cellEligible ? 1 : 0, L.pos, L.atomsByElem,
-        L.es, L.nbrCount, L.nbrCountElem, L.nbrOff, L.key, L.status);
-    nlFinishKernel<<<gWarp, 32 * warpsPerBlock, 0, s>>>(
-        n, L.p, cellEligible ? 1 : 0, L.pos, L.elem, L.nbrOff, L.keyTmp,
-        L.key, L.nbrIdx, L.nbrEl, L.dx, L.dy, L.dz, L.dd, L.status);
-    nlEntryAtomKernel<<<gAtoms, tb, 0, s>>>(n, L.nbrOff, L.entryAtom,
-                                            L.status);
+        L.es, L.nbrCount, L.nbrCountElem, L.nbrOff, out, L.status);
     long const cap = L.capacity;
     int const gE = (int)((cap + tb - 1) / tb);
-    noteLaunches(cellEligible ? 11 : 7);
+    noteLaunches(cellEligible ? 9 : 5);
     nlMirrorKernel<<<gE > 0 ? gE : 1, tb, 0, s>>>(
         n, L.p.nimg, L.elem, L.nbrOff, L.key, L.nbrIdx,
         L.entryAtom, L.mirror, L.status);
@@ -692,7 +761,7 @@ __global__ void nlbPrepareKernel(int n, double const* __restrict__ posIn,
     pos[3 * i + 2] = r[2];
 }
 
-// Warp per atom; MODE 0 counts, MODE 1 writes the (sorted) keys.
+// Warp per atom; MODE 0 counts, MODE 1 writes the entries (in key order).
 template <int MODE>
 __global__ void nlbBruteKernel(int n, int numElements, int NIMG,
                                double const* __restrict__ pos,
@@ -702,7 +771,7 @@ __global__ void nlbBruteKernel(int n, int numElements, int NIMG,
                                int* __restrict__ nbrCount,
                                int* __restrict__ nbrCountElem,
                                int const* __restrict__ nbrOff,
-                               unsigned long long* __restrict__ key,
+                               ListOut const out,
                                int const* __restrict__ status)
 {
     if (status[ST_FLAGS] & FLAG_ABORT) return;
@@ -725,6 +794,7 @@ __global__ void nlbBruteKernel(int n, int numElements, int NIMG,
             long const c = c0 + lane;
             bool hit = false;
             int j = 0, img = 0;
+            double dr[3];
             if (c < ncand)
             {
                 j = structAtoms[eb + (int)(c / nimg)];
@@ -732,16 +802,14 @@ __global__ void nlbBruteKernel(int n, int numElements, int NIMG,
                 int b0, b1, b2;
                 imgDecode(p, img, b0, b1, b2);
                 if (!(j == i && b0 == 0 && b1 == 0 && b2 == 0))
-                {
-                    double dr[3];
                     hit = nlTest(p, ri, pos, j, b0, b1, b2, dr);
-                }
             }
             unsigned const m = __ballot_sync(0xffffffffu, hit);
             if (MODE == 1 && hit)
             {
                 int const off = total + __popc(m & ((1u << lane) - 1u));
-                key[base + off] = nlKey(e, j, img, n, NIMG);
+                writeEntry(out, base + off, i, nlKey(e, j, img, n, NIMG), j,
+                           e, dr);
             }
             total += __popc(m);
             cntE += __popc(m);
@@ -750,51 +818,6 @@ __global__ void nlbBruteKernel(int n, int numElements, int NIMG,
             nbrCountElem[(long)i * numElements + e] = cntE;
     }
     if (MODE == 0 && lane == 0) nbrCount[i] = total;
-}
-
-__global__ void nlbFinishKernel(int n, int NIMG,
-                                double const* __restrict__ pos,
-                                int const* __restrict__ elem,
-                                int const* __restrict__ structOf,
-                                BatchStruct const* __restrict__ bs,
-                                int const* __restrict__ nbrOff,
-                                unsigned long long const* __restrict__ key,
-                                int* __restrict__ nbrIdx,
-                                int8_t* __restrict__ nbrEl,
-                                double* __restrict__ dx,
-                                double* __restrict__ dy,
-                                double* __restrict__ dz,
-                                double* __restrict__ dd,
-                                int const* __restrict__ status)
-{
-    if (status[ST_FLAGS] & FLAG_ABORT) return;
-    int const lane = threadIdx.x & 31;
-    int const i = (int)((blockIdx.x * (long)blockDim.x + threadIdx.x) >> 5);
-    if (i >= n) return;
-    NLParams const& p = bs[structOf[i]].p;
-    long const b = nbrOff[i];
-    int const cnt = nbrOff[i + 1] - nbrOff[i];
-    double const ri[3] = {pos[3 * i], pos[3 * i + 1], pos[3 * i + 2]};
-    unsigned long long const nimg = (unsigned long long)NIMG;
-    for (int t = lane; t < cnt; t += 32)
-    {
-        unsigned long long const k = key[b + t];
-        int const img = (int)(k % nimg);
-        int const j = (int)((k / nimg) % (unsigned long long)n);
-        int b0, b1, b2;
-        imgDecode(p, img, b0, b1, b2);
-        double dr[3];
-        nlTest(p, ri, pos, j, b0, b1, b2, dr);
-        double const n2 = __dadd_rn(__dadd_rn(__dmul_rn(dr[0], dr[0]),
-                                              __dmul_rn(dr[1], dr[1])),
-                                    __dmul_rn(dr[2], dr[2]));
-        nbrIdx[b + t] = j;
-        nbrEl[b + t] = (int8_t)elem[j];
-        dx[b + t] = dr[0];
-        dy[b + t] = dr[1];
-        dz[b + t] = dr[2];
-        dd[b + t] = __dsqrt_rn(n2);
-    }
 }
 
 __global__ void nlbMirrorKernel(int n, int NIMG,
@@ -845,23 +868,10 @@ __global__ void nlbMirrorKernel(int n, int NIMG,
 // outside rc^2 -+ m, where m covers the FP32 rounding of the displacement and
 // image-shift sums (m from a bound on their magnitudes, at least 1e-4 rc^2);
 // between them the exact FP64 test of nlTest does, so the neighbor sets are
-// those of the brute path.  Hits are kept
-// as per-lane image bit masks and placed in key order (lane = j ascending,
-// bits = image ascending) through a warp prefix sum; MODE 0 counts, MODE 1
-// writes the entries.  384 water boxes (101,160 atoms), both passes and
+// those of the brute path.  Hits are kept as per-lane image bit masks and
+// placed in key order (lane = j ascending, bits = image ascending) through a
+// warp prefix sum; MODE 0 counts, MODE 1 writes the entries.  384 water boxes (101,160 atoms), both passes and
 // the entries: 3.7 ms with all 27 images, 1.1 ms so.
-struct LaneOut
-{
-    unsigned long long* key;
-    int*                nbrIdx;
-    int8_t*             nbrEl;
-    double*             dx;
-    double*             dy;
-    double*             dz;
-    double*             dd;
-    int*                entryAtom;
-};
-
 template <int MODE>
 __global__ void __launch_bounds__(256, 4) nlbLaneKernel(int n, int numElements, int NIMG,
                               double const* __restrict__ pos,
@@ -871,7 +881,7 @@ __global__ void __launch_bounds__(256, 4) nlbLaneKernel(int n, int numElements, 
                               int const* __restrict__ structAtoms,
                               int* __restrict__ nbrCount,
                               int* __restrict__ nbrCountElem,
-                              int const* __restrict__ nbrOff, LaneOut const out,
+                              int const* __restrict__ nbrOff, ListOut const out,
                               int const* __restrict__ status)
 {
     if (status[ST_FLAGS] & FLAG_ABORT) return;
@@ -1050,12 +1060,12 @@ void launchNeighborListBatch(NLBatchLaunch const& L, cudaStream_t s)
                                            L.normalize, L.convLength, L.pos);
     long const cap = L.capacity;
     int const gE = (int)((cap + tb - 1) / tb);
+    ListOut const out{L.key, L.nbrIdx, L.nbrEl, L.dx, L.dy, L.dz, L.dd,
+                      L.entryAtom};
     // Structures with more than 128 images (boxes below rc / 2) take the
     // plain brute path.
     if (L.NIMG <= 128)
     {
-        LaneOut const out{L.key, L.nbrIdx, L.nbrEl, L.dx, L.dy, L.dz, L.dd,
-                          L.entryAtom};
         nlbLaneKernel<0><<<gWarp, 32 * wpb, 0, s>>>(
             n, L.numElements, L.NIMG, L.pos, L.structOf, L.bs, L.one,
             L.structAtoms, L.nbrCount, L.nbrCountElem, L.nbrOff, out,
@@ -1079,18 +1089,13 @@ void launchNeighborListBatch(NLBatchLaunch const& L, cudaStream_t s)
     }
     nlbBruteKernel<0><<<gWarp, 32 * wpb, 0, s>>>(
         n, L.numElements, L.NIMG, L.pos, L.structOf, L.bs, L.structAtoms,
-        L.nbrCount, L.nbrCountElem, L.nbrOff, L.key, L.status);
+        L.nbrCount, L.nbrCountElem, L.nbrOff, out, L.status);
     nlScanKernel<<<1, 1024, 0, s>>>(n, L.nbrCount, L.nbrOff, L.capacity,
                                     L.status);
     nlbBruteKernel<1><<<gWarp, 32 * wpb, 0, s>>>(
         n, L.numElements, L.NIMG, L.pos, L.structOf, L.bs, L.structAtoms,
-        L.nbrCount, L.nbrCountElem, L.nbrOff, L.key, L.status);
-    nlbFinishKernel<<<gWarp, 32 * wpb, 0, s>>>(
-        n, L.NIMG, L.pos, L.elem, L.structOf, L.bs, L.nbrOff, L.key,
-        L.nbrIdx, L.nbrEl, L.dx, L.dy, L.dz, L.dd, L.status);
-    nlEntryAtomKernel<<<gAtoms, tb, 0, s>>>(n, L.nbrOff, L.entryAtom,
-                                            L.status);
-    noteLaunches(7);
+        L.nbrCount, L.nbrCountElem, L.nbrOff, out, L.status);
+    noteLaunches(5);
     nlbMirrorKernel<<<gE > 0 ? gE : 1, tb, 0, s>>>(
         n, L.NIMG, L.elem, L.structOf, L.bs, L.nbrOff, L.key, L.nbrIdx,
         L.entryAtom, L.mirror, L.status);

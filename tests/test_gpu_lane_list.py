@@ -125,10 +125,10 @@ def test_batch_equals_single(gpu):
         e0 += m
 
 
-@pytest.mark.parametrize("mol", [512, 513])
+@pytest.mark.parametrize("mol", [213, 214, 512, 513])
 def test_both_sides_of_the_rule(gpu, mol):
-    """1,536 and 1,539 atoms: one structure on the lane path, one on the cell
-    path; both as the same structure in a batch of one."""
+    """639 and 642 atoms: one structure on the lane path, one on the cell
+    path (1,536 and 1,539 too); all as the same structure in a batch of one."""
     box, pos, elem = synth.water_box(mol, 3)
     p, q = _prediction(), _prediction()
     p.set_structure(pos, elem, box)
