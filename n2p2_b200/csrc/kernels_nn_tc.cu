@@ -3,7 +3,7 @@
 // NeuralNetwork::calculateDEdG (:396-442) for 128 atoms of one element at a
 // time.
 //
-// One CTA (4 warps, persistent over tiles) per SM.  Per tile:
+// One CTA (16 warps, persistent over tiles) per SM.  Per tile:
 //   forward   z_l = W_l h_{l-1} + b_l   as D[128 x out] = A[128 x in] B^T with
 //             B = W_l (out x in, K-major), one tcgen05.mma per 16 of K;
 //   output    E = f_out(w . h_H + b)    FP32 dot product in the epilogue;
@@ -13,9 +13,13 @@
 // without swizzle (8-row x 16-byte core matrices; LBO = 128 B between the
 // two K halves of an MMA step, SBO = K * 16 B between 8-row groups);
 // accumulators are FP32 in tensor memory (row = lane, column = neuron).
-// Thread r of the CTA owns row (atom) r: it reads its accumulator row with
-// tcgen05.ld, applies bias and activation in FP32, keeps f' in shared memory
-// for the backward sweep and writes the next layer's BF16 operand row.
+// Warps w, w + 4, w + 8 and w + 12 own the rows (atoms) of lane quarter w and
+// take every fourth block of 16 columns of them: they read the accumulators
+// with tcgen05.ld, apply bias and activation in FP32, keep f' in tensor
+// memory for the backward sweep and write the next layer's BF16 operands.
+// Bound by these epilogues (192 activations a row for 92-64-64-64-1, the MMAs
+// are a few percent), hence the 16 warps: 98,304 atoms 0.73 ms with 4 warps a
+// CTA, 0.40 with 8, 0.26 with 16.
 // One elected thread issues the MMAs and commits them to an mbarrier; every
 // wait is bounded and reports FLAG_TC_TIMEOUT instead of hanging.
 //
@@ -37,7 +41,8 @@ namespace n2p2b
 namespace
 {
 
-constexpr int kTcThreads = 128;
+constexpr int kTcGroups = 4;               // warps that share a row
+constexpr int kTcThreads = 128 * kTcGroups;
 constexpr long kWaitLimit = 1L << 22;     // try_wait rounds before giving up
 constexpr float kExpLimitF = 35.0f;       // EXP_LIMIT, NeuralNetwork.cpp:25
 
@@ -378,13 +383,15 @@ nnTcKernel(__grid_constant__ TcNNParams const P,
     __syncthreads();
     tcFenceAfter();
     uint32_t const tmem = *sTmem;
-    uint32_t const tRow = tmem + ((uint32_t)(warp * 32) << 16);
+    uint32_t const tRow = tmem + ((uint32_t)((warp & 3) * 32) << 16);
     uint32_t const aH = smemAddr(sAh);
     uint32_t const aL = P.split ? smemAddr(sAl) : aH;
     uint32_t phase = 0;
     int loaded = -1;
     bool ok = true;
-    int const r = tid;
+    int const r = tid & (kTcRows - 1);
+    int const cFirst = (warp >> 2) * 16;       // this warp's column blocks
+    constexpr int cStep = 16 * kTcGroups;
 
     for (int tile = blockIdx.x; tile < total && ok; tile += gridDim.x)
     {
@@ -409,11 +416,13 @@ nnTcKernel(__grid_constant__ TcNNParams const P,
         bool const valid = row0 + r < rowEnd;
         int const atom = valid ? L.atomsByElem[row0 + r] : -1;
 
-        // Input tile: scaled symmetry functions as BF16 (warp w loads rows
-        // 32w .. 32w + 31, lanes over columns).
-        for (int rr = 0; rr < 32; ++rr)
+        // Input tile: scaled symmetry functions as BF16 (rows over warps,
+        // lanes over columns).
+        constexpr int kRowsPerWarp = kTcRows / (kTcThreads / 32);
+#pragma unroll 4
+        for (int rr = 0; rr < kRowsPerWarp; ++rr)
         {
-            int const row = warp * 32 + rr;
+            int const row = warp * kRowsPerWarp + rr;
             int const at = (row0 + row < rowEnd) ? L.atomsByElem[row0 + row]
                                                  : -1;
             for (int k = lane; k < N.ninP; k += 32)
@@ -439,7 +448,7 @@ nnTcKernel(__grid_constant__ TcNNParams const P,
             if (!ok) break;
             float const* b = sF + Ly.b;
             bool const last = (l == N.hidden - 1);
-            for (int c0 = 0; c0 < Ly.outP; c0 += 16)
+            for (int c0 = cFirst; c0 < Ly.outP; c0 += cStep)
             {
                 float v[16], d[16];
                 tmemLd16(tRow + c0, v);
@@ -465,15 +474,24 @@ nnTcKernel(__grid_constant__ TcNNParams const P,
             tmemWaitSt();
         }
         if (!ok) break;
+        // Sum over the row's warps (the operand tile is free: the last GEMM
+        // has read it).
+        float* const part = reinterpret_cast<float*>(sAh);
+        part[(warp >> 2) * kTcRows + r] = eAcc;
+        __syncthreads();
+        eAcc = 0.0f;
+#pragma unroll
+        for (int g = 0; g < kTcGroups; ++g) eAcc += part[g * kTcRows + r];
+        __syncthreads();
         float E, dEz;
         actF(N.outAct, eAcc + sF[N.outB], E, dEz);
-        if (valid) L.energy[atom] = (double)E;
+        if (valid && tid < kTcRows) L.energy[atom] = (double)E;
         if (!L.derivatives) continue;
 
         // Backward sweep.
         {
             TcLayer const& LH = N.layer[N.hidden - 1];
-            for (int c0 = 0; c0 < LH.outP; c0 += 16)
+            for (int c0 = cFirst; c0 < LH.outP; c0 += cStep)
             {
                 float v[16];
                 tmemLd16(tRow + LH.fp + c0, v);
@@ -493,7 +511,7 @@ nnTcKernel(__grid_constant__ TcNNParams const P,
             if (l > 0)
             {
                 TcLayer const& Lp = N.layer[l - 1];
-                for (int c0 = 0; c0 < Ly.inP; c0 += 16)
+                for (int c0 = cFirst; c0 < Ly.inP; c0 += cStep)
                 {
                     float v[16], d[16];
                     tmemLd16(tRow + c0, v);
@@ -507,11 +525,25 @@ nnTcKernel(__grid_constant__ TcNNParams const P,
             else
             {
                 float* o = L.dEdG + (long)(valid ? atom : 0) * L.maxSF;
-                for (int c0 = 0; c0 < Ly.inP; c0 += 16)
+                for (int c0 = cFirst; c0 < Ly.inP; c0 += cStep)
                 {
                     float v[16];
                     tmemLd16(tRow + c0, v);
-                    if (valid)
+                    if (!valid) continue;
+                    if ((L.maxSF & 3) == 0)
+                    {
+#pragma unroll
+                        for (int q = 0; q < 16; q += 4)
+                            if (c0 + q + 3 < N.nin)
+                                *reinterpret_cast<float4*>(o + c0 + q) =
+                                    make_float4(v[q], v[q + 1], v[q + 2],
+                                                v[q + 3]);
+                            else
+#pragma unroll
+                                for (int k = q; k < q + 4; ++k)
+                                    if (c0 + k < N.nin) o[c0 + k] = v[k];
+                    }
+                    else
                     {
 #pragma unroll
                         for (int q = 0; q < 16; ++q)

@@ -111,3 +111,28 @@ def test_networks(gpu, tmp_path, name, precision, norm, mol):
         en, de, ee, ed = _network(_layers(d, z, nsf), G[a, :nsf], norm, u)
         assert np.all(np.abs(E[a] - en) <= ee)
         assert np.all(np.abs(D[a, :nsf] - de) <= ed)
+
+
+@pytest.mark.parametrize("mol", [11, 43, 1500])
+@pytest.mark.parametrize("name", ["h2o_52", "h2o_92", "h2o_wtd"])
+def test_tensor_core_networks(gpu, name, mol):
+    """Rows shared by four warps (tensor cores): less than a tile, a tile
+    and one atom, many; 16-byte and single stores of dE/dG.  Operands are
+    pairs of BF16: a product errs by less than 2^-16 of itself."""
+    from n2p2_b200.mode import Prediction
+    d = os.path.join(POTS, name)
+    p = Prediction(d)
+    p.setup()
+    p.setup_symmetry_function_statistics(False, False, False, False)
+    p.set_precision("mixed")
+    box, pos, elem = synth.water_box(mol, 3)
+    p.set_structure(pos, elem, box)
+    p.evaluate_nnp(True)
+    G, E, D = p.symmetry_functions(), p.atomic_energies(), p.dEdG()
+    for e, z in enumerate((1, 8)):
+        nsf = p.num_symmetry_functions(e)
+        a = np.flatnonzero(np.asarray(elem) == e)
+        en, de, ee, ed = _network(_layers(d, z, nsf), G[a, :nsf], False,
+                                  2.0 ** -16)
+        assert np.all(np.abs(E[a] - en) <= ee)
+        assert np.all(np.abs(D[a, :nsf] - de) <= ed)
