@@ -42,7 +42,7 @@ namespace
 {
 
 constexpr int kGradRows = 64;
-constexpr int kGradThreads = 128;
+constexpr int kGradThreads = 512;
 
 __global__ void residualKernel(StudentLaunch const L)
 {
@@ -65,9 +65,12 @@ __global__ void residualKernel(StudentLaunch const L)
 // Warp per atom j: u_j over its symmetry functions, lanes over the entries.
 // Bound by reading dG/dr once: the entries' residual differences are gathered
 // once per block of 32 kAdjEntries entries and stay in registers, then the
-// rows of kAdjSlots slots are read together (6,144 atoms, 437 MB: 0.297 ms
-// with the gather inside the slot loop and one slot at a time).
-constexpr int kAdjEntries = 4, kAdjSlots = 2;
+// rows of kAdjSlots slots are read together and their lane sums reduced
+// together, half of them by each half of the warp at every step (9 shuffles
+// for 8 sums).  6,144 atoms, 437 MB: 0.297 ms with the gather inside the slot
+// loop and one slot at a time, 0.204 with two slots and a full reduction
+// each, 0.164 so.
+constexpr int kAdjEntries = 4, kAdjSlots = 8;
 
 template <typename T>
 __global__ void __launch_bounds__(128)
@@ -142,12 +145,24 @@ adjointKernel(StudentLaunch const L)
                                       + qz[k] * (float)row[2 * cnt + 32 * k];
                     }
 #pragma unroll
-                    for (int c = 0; c < kAdjSlots; ++c)
+                    for (int h = kAdjSlots / 2; h >= 1; h >>= 1)
                     {
-                        if (sl + c >= ns) break;
-                        v[c] = warpSumF(v[c]);
-                        if (lane == 0) acc[tab[sl + c]] += v[c];
+                        // h = 4, 2, 1: lane bits 16, 8, 4 choose the slots.
+                        int const bit = 4 * h;
+                        bool const up = (lane & bit) != 0;
+#pragma unroll
+                        for (int c = 0; c < h; ++c)
+                        {
+                            float const keep = up ? v[c + h] : v[c];
+                            float const give = up ? v[c] : v[c + h];
+                            v[c] = keep + __shfl_xor_sync(0xffffffffu, give,
+                                                          bit);
+                        }
                     }
+                    v[0] += __shfl_xor_sync(0xffffffffu, v[0], 2);
+                    v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
+                    int const mine = sl + (lane >> 2);
+                    if ((lane & 3) == 0 && mine < ns) acc[tab[mine]] += v[0];
                 }
                 __syncwarp();
             }
@@ -159,7 +174,10 @@ adjointKernel(StudentLaunch const L)
     }
 }
 
-// Partial gradients of 64 atoms of one element per block.
+// Partial gradients of 64 atoms of one element per block, a thread per (row,
+// neuron) and then per weight: serial sums over inputs and rows, so the time
+// is their number per thread (6,144 atoms, 92-32-1: 0.096 ms with 128
+// threads, 0.040 with 512).
 template <typename T>
 __global__ void __launch_bounds__(kGradThreads)
 gradKernel(StudentLaunch const L)
