@@ -175,11 +175,31 @@ void launchPair(int pass, SFParams const& P, PairParams const& host,
 {
     if (L0.n <= 0) return;
     PairLaunch L = L0;
-    // A warp per atom once there are atoms for all of them and three blocks
-    // per multiprocessor fit.
+    // One or four warps per atom.  One needs no barriers and adds no shares,
+    // four keep the chip busy with fewer atoms and need a quarter of the
+    // shared memory.  One if three blocks per multiprocessor fit (where they
+    // do not, 2,048 atoms of anisole, one / four: values 4.1 / 1.6 ms, forces
+    // 9.6 / 3.6) and:
+    //  values  its warps fill two thirds of a wave, but do not just begin a
+    //          second one (52 functions, FP64, one / four: 768 atoms 0.070 /
+    //          0.062 ms, 1,200 0.080 / 0.086, 1,920 0.132 / 0.115, 3,072
+    //          0.154 / 0.168, 24,576 0.97 / 1.16);
+    //  forces  enough waves to even out the atoms' unequal work (FP64: 6,000
+    //          atoms 0.68 / 0.64, 9,000 0.92 / 0.94, 24,576 2.41 / 2.52; FP32,
+    //          92 functions: 4,200 0.357 / 0.351, 6,000 0.477 / 0.488);
+    //          atoms of few neighbors have too few items of eight owners for
+    //          four warps (1,728 atoms of Cu2S 0.267 / 0.308).
     L.wpa = 1;
     std::size_t shm = layout(host, L, pass);
-    if (3 * (shm + 1024) > kSmemSM || L.n < 12 * L.sms)
+    bool const f = L.precision != PREC_FP64;
+    std::size_t const blocks = std::min<std::size_t>(
+        f ? 4 : 3, kSmemSM / (shm + 1024));
+    double const waves = (double)L.n
+                       / ((double)(kWarpsPerCta * std::max<std::size_t>(blocks, 1))
+                          * L.sms);
+    bool one = waves >= 2.0 / 3.0 && (waves <= 1.0 || waves >= 1.3);
+    if (pass == 1 && L.cap > 80) one = L.n >= (f ? 36 : 48) * L.sms;
+    if (blocks < 3 || !one)
     {
         L.wpa = kWarpsPerCta;
         shm = layout(host, L, pass);

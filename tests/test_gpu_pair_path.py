@@ -179,3 +179,24 @@ def test_mixed(gpu, monkeypatch, pot):
                                                                  box)
     assert abs(e1 - e0) / len(elem) <= 1e-4
     assert np.sqrt(np.mean((f1 - f0) ** 2)) <= 5e-3
+
+
+@pytest.mark.parametrize("mol", [394, 395, 592, 593, 769, 770])
+def test_team_sizes(gpu, monkeypatch, mol):
+    """Atom counts on both sides of the values pass's rules (two thirds of a
+    wave, one wave, 1.3 waves of 148 x 12 warps) against one and four warps
+    per atom asked for."""
+    box, pos, elem = synth.water_box(mol, 4)
+    out = []
+    for wpa in (None, "1", "4"):
+        if wpa is None:
+            monkeypatch.delenv("N2P2B_PAIR_WPA", raising=False)
+        else:
+            monkeypatch.setenv("N2P2B_PAIR_WPA", wpa)
+        p = _prediction(os.path.join(GOLD, POTS[0]), False, monkeypatch)
+        p.set_structure(pos, elem, box)
+        p.evaluate_nnp(True)
+        out.append((p.symmetry_functions(), p.forces()))
+    for G, F in out[1:]:
+        assert np.abs(out[0][0] - G).max() <= 1e-12 * np.abs(G).max()
+        assert np.abs(out[0][1] - F).max() <= 1e-10 * np.abs(F).max()
