@@ -870,19 +870,21 @@ __global__ void nlbMirrorKernel(int n, int NIMG,
 // between them the exact FP64 test of nlTest does, so the neighbor sets are
 // those of the brute path.  Hits are kept as per-lane image bit masks and
 // placed in key order (lane = j ascending, bits = image ascending) through a
-// warp prefix sum; MODE 0 counts, MODE 1 writes the entries.  384 water boxes (101,160 atoms), both passes and
-// the entries: 3.7 ms with all 27 images, 1.1 ms so.
+// warp prefix sum; MODE 0 counts, MODE 1 writes the entries.  384 water boxes
+// (101,160 atoms), both passes and the entries: 3.7 ms with all 27 images,
+// 1.1 ms so.
 template <int MODE>
-__global__ void __launch_bounds__(256, 4) nlbLaneKernel(int n, int numElements, int NIMG,
-                              double const* __restrict__ pos,
-                              int const* __restrict__ structOf,
-                              BatchStruct const* __restrict__ bs,
-                              __grid_constant__ BatchStruct const one,
-                              int const* __restrict__ structAtoms,
-                              int* __restrict__ nbrCount,
-                              int* __restrict__ nbrCountElem,
-                              int const* __restrict__ nbrOff, ListOut const out,
-                              int const* __restrict__ status)
+__global__ void __launch_bounds__(256, 4)
+nlbLaneKernel(int n, int numElements, int NIMG,
+              double const* __restrict__ pos,
+              int const* __restrict__ structOf,
+              BatchStruct const* __restrict__ bs,
+              __grid_constant__ BatchStruct const one,
+              int const* __restrict__ structAtoms,
+              int* __restrict__ nbrCount,
+              int* __restrict__ nbrCountElem,
+              int const* __restrict__ nbrOff, ListOut const out,
+              int const* __restrict__ status)
 {
     if (status[ST_FLAGS] & FLAG_ABORT) return;
     int const lane = threadIdx.x & 31;

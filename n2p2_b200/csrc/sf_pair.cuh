@@ -14,18 +14,27 @@
 // members.  Compact functions have the same form (run = radial window
 // functions, shape = window function of theta).
 //
-// Values pass: CTA per atom; each unordered triplet once.  Warps walk the
-// rows (j, k > j) of a unit, test r_jk with the lane on k and push the valid
-// pairs into a 64-entry queue per warp, from which full warps of triplets
-// are evaluated (97 % of the lanes busy); the unit's sums stay in registers
-// (lane sums, then one fixed-order reduction per unit).
+// Both passes: a team of one or four warps per atom (launchPair says when).
 //
-// Forces pass: CTA per atom; an item is eight owners j of one element on
-// four lanes each, owners ordered by their partner counts so that the
-// owners of an item have similar trip counts.  The item's lanes build the
-// owners' partner lists from the validity mask, walk the units with the
-// unit's parameters the same for the whole warp, and add the four slices
-// at the end.  Each pair term has one writer: no atomics, fixed order.
+// Values pass: each unordered triplet once.  Lanes own the rows of the
+// validity mask (r_jk < rc) and list their rows' valid pairs; the team walks
+// the list 32 pairs at a time; the unit's sums stay in registers (lane sums,
+// then one fixed-order reduction per unit).
+//
+// Forces pass: an item is eight owners j of one element on four lanes each,
+// owners ordered by their partner counts so that the owners of an item have
+// similar trip counts.  The item's lanes build the owners' partner lists
+// from the validity mask, walk the units with the unit's parameters the same
+// for the whole warp, and add the four slices at the end.  Each pair term
+// has one writer: no atomics, fixed order.
+//
+// Bounds.  Memory is small (the neighbor entries once per pass, 24 B written
+// per entry); the FP64 instructions (about 80 a triplet for the values, 130
+// per owner for the forces, 3 runs x 4 shapes) and their latency at 12 to 16
+// warps per multiprocessor bound both passes.  24,576 water atoms, 52
+// functions, FP64: 0.96 + 2.4 ms, where dG/dr took 6.1 to form and 0.4 to
+// contract (2 GB each way); 98,304 atoms, 92 functions, FP32: 2.7 + 6.8 ms
+// against 25.1 + 1.5.
 #pragma once
 
 #include "sf_impl.cuh"
@@ -1144,8 +1153,10 @@ __device__ __forceinline__ void pow2ValuesN(SFParams const& P, UnitTables const&
     default: pow2Values<R, CT, NZ, 4, MASK, NARROW>(P, tb, u, w); break;
     }
 }
-// The sets {1}, {1, 4}, {1, 2, 4} and {1, 2, 4, 16} of zeta are compiled without tests of the slots (a test is a branch, which keeps the
-// compiler from overlapping the slots' work with the exponentials'); other sets test them.
+// The sets {1}, {1, 4}, {1, 2, 4} and {1, 2, 4, 16} of zeta are compiled
+// without tests of the slots (a test is a branch, which keeps the compiler
+// from overlapping the slots' work with the exponentials'); other sets test
+// them.
 template <typename R, int CT, int NZ, bool SETS>
 __device__ __forceinline__ void pow2ValuesNarrow(SFParams const& P, UnitTables const& tb,
     PairUnit const& u, Walk<R> const& w)
@@ -1782,8 +1793,9 @@ __device__ __forceinline__ void pow2ForcesN(SFParams const& P, UnitTables const&
     default: pow2Forces<R, CT, NZ, 4, MASK, NARROW>(P, tb, u, C, W, p, o); break;
     }
 }
-// The sets {1}, {1, 4}, {1, 2, 4} and {1, 2, 4, 16} of zeta are compiled without tests of the slots (52 functions,
-// 6,144 atoms, FP64: 0.90 -> 0.71 ms); other sets test them.
+// The sets {1}, {1, 4}, {1, 2, 4} and {1, 2, 4, 16} of zeta are compiled
+// without tests of the slots (52 functions, 6,144 atoms, FP64: 0.90 -> 0.71
+// ms); other sets test them.
 template <typename R, int CT, int NZ, bool SETS>
 __device__ __forceinline__ void pow2ForcesNarrow(SFParams const& P, UnitTables const& tb,
     PairUnit const& u, R const* C, Staged<R> const& W, Partners const& p,
