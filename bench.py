@@ -11,14 +11,15 @@ uniform O positions with O-O >= 4.7 bohr, seeded orientations, then 100
 frames with Gaussian position noise sigma = 0.1 bohr.  Potential: 52 symmetry
 functions per element (radial + narrow angular, cos cutoff 12 bohr), NN
 52-25-25-1 (tanh), seeded Nguyen-Widrow weights (tests/golden/potentials/
-h2o_52).  One step = one frame through neighbor list, symmetry functions +
-dG/dr, atomic NNs + dE/dG, energy and forces, all in FP64.
+h2o_52).  One step = one frame through neighbor list, symmetry functions,
+atomic NNs + dE/dG, energy and forces (dE/dG contracted with the
+symmetry-function derivatives inside the triplets), all in FP64.
 
 Metric: E+F atoms/s (higher is better).
   value : device-resident frames (HBM), K steps between CUDA events on the
           library's stream, max over ranks; frames cycle through 100
-          distinct coordinate sets and the per-frame working set (dG/dr,
-          2 GB) is far larger than L2.
+          distinct coordinate sets and the per-frame working set (neighbor
+          entries and pair forces, 0.2 GB) is larger than L2.
   e2e   : the same through the C-ABI with HOST buffers -- every step copies
           the frame's positions host->device (pinned) and reads back energy
           and forces (n2p2b_set_positions / n2p2b_evaluate /
@@ -74,29 +75,14 @@ POT_DIR = os.path.join(ROOT, "tests", "golden", "potentials")
 POT = os.path.join(POT_DIR, "h2o_52")
 STAGES = ("neighbor_list", "symmetry_functions", "neural_networks", "energy",
           "forces")
-# DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) of one FP64
-# symmetry-function launch on this workload, per kernel family, from the
-# ncu captures summarized under profiles/ (12,288-atom box), scaled to the
-# 24,576-atom frame by its neighbor entries (x 2.002): the staged-triplet
-# kernel (variants 6, 7; the default) and the per-owner kernel (0-5).
-SF_TRAFFIC = {
-    "staged": (2.669e9, "ncu dram__bytes_read.sum + dram__bytes_write.sum of "
-                        "the FP64 sfStagedKernel on the 12,288-atom box "
-                        "(1.333 GB), x 2.002 neighbor entries for 24,576 "
-                        "atoms (profiles/sfStagedKernel_fp64_fp32_"
-                        "water12288.md)"),
-    "owner": (4.184e9, "ncu dram__bytes_read.sum + dram__bytes_write.sum of "
-                       "the FP64 per-owner sfKernel on the 12,288-atom box "
-                       "(2.090 GB), x 2.002 neighbor entries for 24,576 "
-                       "atoms (profiles/sfKernel_fp64_fp32_water12288.md)"),
-}
-
-
-def sf_family(tune: str) -> str:
-    """Kernel family of the autotuner's choice ("... sf variant N ...")."""
-    import re
-    m = re.search(r"sf variant (\d+)", tune or "")
-    return "staged" if m and int(m.group(1)) >= 6 else "owner"
+# DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) of the FP64
+# symmetry-function kernels (values and forces) on this workload, from the ncu
+# capture summarized under profiles/ (12,288-atom box), scaled to the
+# 24,576-atom frame by its neighbor entries (x 2.002).
+SF_TRAFFIC = (1.850e8, "ncu dram__bytes_read.sum + dram__bytes_write.sum of the "
+              "FP64 pairValueKernel and pairTermKernel on the 12,288-atom box "
+              "(0.0924 GB), x 2.002 neighbor entries for 24,576 atoms "
+              "(profiles/pairKernels_fp64_fp32_water12288.md)")
 
 
 N_MOL = 8192
@@ -154,7 +140,8 @@ def config(n_gpus: int, steps_note: str = ""):
                      "angular G3, cos cutoff rc = 12 bohr), NN 52-25-25-1 tanh",
         "form": "plain FP64",
         "atoms_per_step_per_gpu": 3 * N_MOL,
-        "l2": "per-frame working set > L2 (dG/dr buffer ~2 GB; frames cycle)",
+        "l2": "per-frame working set > L2 (neighbor entries and pair forces "
+              "~0.2 GB; frames cycle)",
         "parallelism": f"replicas x{n_gpus}",
         **({"note": steps_note} if steps_note else {}),
     }
@@ -246,8 +233,11 @@ def potential_shape(p):
 def work_model(cnt, dr, d, shape, mac, rc=12.0):
     """Exact neighbor (n) and valid-triplet (T) counts of one frame and the
     FLOP / byte model: per triplet 40 + 60 M_a, per (pair, radial member)
-    20, NN 3*2*MAC, chain rule 6 per stored Vec3D slot; bytes of the SF
-    kernel = neighbor data read + dG/dr, G and dG/dr(self) written."""
+    20, NN 3*2*MAC, chain rule 6 per Vec3D slot.  The FLOPs are those of the
+    plain formulation (dG/dr of every member, then the chain rule); the
+    kernels contract dE/dG inside the triplets and execute fewer.  Bytes of
+    the two symmetry-function kernels = neighbor data read twice, G written,
+    dE/dG read, pair and self terms written."""
     import torch
     M_a, M_r, S, n_sf = shape
     dev = torch.device("cuda")
@@ -274,7 +264,7 @@ def work_model(cnt, dr, d, shape, mac, rc=12.0):
     n = int(cnt.sum())
     flops_sf = T * (40 + 60 * M_a) + n * M_r * 20
     flops_all = flops_sf + N * 3 * 2 * mac + 6 * (n * S + N * n_sf)
-    bytes_sf = n * 32 + n * S * 3 * 8 + N * n_sf * 8 * 4 + N * 8 * 2
+    bytes_sf = n * (2 * 32 + 24) + N * n_sf * 8 * 2 + N * 24
     return {"atoms": N, "neighbors": n, "triplets": T,
             "neighbors_per_atom": n / N, "triplets_per_atom": T / N,
             "M_a": M_a, "M_r": M_r, "S": S, "n_sf": n_sf, "mac_nn": mac,
@@ -848,13 +838,13 @@ def run_ours(a):
         rep.close()
         return
 
-    # ---- roofline of the dominant kernel (symmetry functions) -------------
+    # ---- roofline of the symmetry-function kernels (values, forces) -------
     p.set_positions(dev_frames[0])
     p.evaluate_nnp(True)
     cnt, index, dr, d = p.neighbor_list()
     mac = 52 * 25 + 25 * 25 + 25
     wm = work_model(cnt, dr, d, potential_shape(p), mac)
-    sf_s = per[1] / 1e3
+    sf_s = (per[1] + per[4]) / 1e3
     hbm_peak, peak_kind = measured_peaks()
     gbs = wm["bytes_sf"] / sf_s / 1e9
     fp64_peak = fp64_peak_tflops()
@@ -876,9 +866,8 @@ def run_ours(a):
         "stage_ms_per_step": dict(zip(STAGES, per)),
         "autotune": tune,
         "roofline": {
-            "kernel": ("sfStagedKernel<double>" if sf_family(tune) == "staged"
-                       else "sfKernel<double>")
-                      + " (symmetry functions + dG/dr)",
+            "kernel": "pairValueKernel<double> + pairTermKernel<double> "
+                      "(symmetry functions; their force terms)",
             "bound": "fp64",
             "achieved": sf_tflops, "peak": fp64_peak, "unit": "TFLOP/s",
             "frac": sf_tflops / fp64_peak,
@@ -887,10 +876,12 @@ def run_ours(a):
                            "no FP64 figure)",
             "achieved_source": "counting-model FLOPs of the frame (exact "
                                "triplet and neighbor counts, see work) / "
-                               "the SF stage's CUDA-event time",
+                               "the CUDA-event time of the SF and force "
+                               "stages; the kernels execute fewer "
+                               "(dE/dG is contracted in the triplets)",
             "algorithmic_flops_per_launch": wm["flops_sf"],
-            "traffic": SF_TRAFFIC[sf_family(tune)][0],
-            "traffic_source": SF_TRAFFIC[sf_family(tune)][1],
+            "traffic": SF_TRAFFIC[0],
+            "traffic_source": SF_TRAFFIC[1],
             "hbm": {"achieved": gbs, "peak": hbm_peak, "unit": "GB/s",
                     "frac": gbs / hbm_peak,
                     "peak_source": f"{peak_kind} (MEASURED_PEAKS.json "
