@@ -240,6 +240,7 @@ nnKernel(__grid_constant__ NNParams const P, NNLaunch const L)
 // each sum runs over the inputs in the same order as above.  For many atoms
 // only: a warp's chain of layers takes as long as the per-atom kernel's.
 constexpr int kNNTile = 4;
+constexpr int kNNTileSmem = 56 * 1024;
 
 struct NNTileLaunch
 {
@@ -690,7 +691,7 @@ void launchNNTile(NNParams const& P, NNTileLaunch const& N, int blocks,
 {
     cudaFuncSetAttribute(nnTileKernel<T>,
                          cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)shm);
+                         kNNTileSmem);  // one value: threads share it
     nnTileKernel<T><<<blocks, 32 * kNNWarps, shm, s>>>(P, N);
 }
 
@@ -723,7 +724,7 @@ void launchNeuralNetworks(NNParams const& P, NNLaunch const& L,
         bool const f32 = L.precision != PREC_FP64;
         std::size_t const shm = (f32 ? sizeof(float) : sizeof(double))
                               * (std::size_t)kNNWarps * N.stride;
-        if (shm <= 56 * 1024)
+        if (shm <= (std::size_t)kNNTileSmem)
         {
             int const blocks = (N.warpBeg[kMaxElem] + kNNWarps - 1) / kNNWarps;
             noteLaunches(1);

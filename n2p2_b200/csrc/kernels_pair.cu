@@ -44,7 +44,7 @@ namespace
 
 constexpr int kWarpsPerCta = 4, kOwnersPerItem = 8;
 
-constexpr std::size_t kSmemBlock = 227 * 1024, kSmemSM = 228 * 1024;
+constexpr std::size_t kSmemSM = 228 * 1024;
 
 // Shared-memory layout of a pass (0 values, 1 forces) with L.wpa warps per
 // atom; returns its bytes.
@@ -166,8 +166,8 @@ bool pairFits(PairParams const& T, int cap, int precision, int maxSF)
     L.precision = precision;
     L.maxSF = maxSF;
     L.wpa = kWarpsPerCta;
-    return cap < 65536 && layout(T, L, 0) <= kSmemBlock
-        && layout(T, L, 1) <= kSmemBlock;
+    return cap < 65536 && layout(T, L, 0) <= (std::size_t)kPairSmemBlock
+        && layout(T, L, 1) <= (std::size_t)kPairSmemBlock;
 }
 
 void launchPair(int pass, SFParams const& P, PairParams const& host,

@@ -38,6 +38,9 @@ constexpr int kPairCompRuns = 9;      // compact units
 constexpr int kPairCompShapes = 6;
 constexpr int kPairMaxRc = 4;         // (cutoff radius, weighted) per element
 constexpr int kPairMaxRad = 16;       // radial window functions per element
+// Dynamic shared memory of a block, at most: 227 KB less 1 KB for the
+// kernels' static arrays.
+constexpr int kPairSmemBlock = 226 * 1024;
 
 struct PairUnit
 {

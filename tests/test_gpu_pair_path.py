@@ -200,3 +200,32 @@ def test_team_sizes(gpu, monkeypatch, mol):
     for G, F in out[1:]:
         assert np.abs(out[0][0] - G).max() <= 1e-12 * np.abs(G).max()
         assert np.abs(out[0][1] - F).max() <= 1e-10 * np.abs(F).max()
+
+
+def test_two_threads(gpu, monkeypatch):
+    """Two host threads whose launches of the same kernels take different
+    amounts of shared memory: results as alone."""
+    import threading
+    work = []
+    for mol, scale in ((64, 1.0), (64, 0.85)):
+        box, pos, elem = synth.water_box(mol, 6)
+        p = _prediction(os.path.join(GOLD, POTS[0]), False, monkeypatch)
+        p.set_structure(pos * scale, elem, box * scale)
+        p.evaluate_nnp(True)
+        work.append((p, p.forces()))
+    wrong = []
+
+    def run(p, f0):
+        try:
+            for _ in range(50):
+                p.evaluate_nnp(True)
+                if not np.array_equal(p.forces(), f0):
+                    wrong.append("forces")
+        except Exception as e:        # noqa: BLE001
+            wrong.append(repr(e))
+    threads = [threading.Thread(target=run, args=w) for w in work]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong
