@@ -965,7 +965,8 @@ __device__ __forceinline__ void pow2Values(SFParams const& P,
             }
         }
     });
-    flushCells<R, NZ * NR * 2>(w, acc, u.cell, 2 * NZ * NR);
+    // Slots the unit does not have hold zeros and have no cells.
+    flushCells<R, NZ * NR * 2>(w, acc, u.cell, pairUnitCells(u));
 }
 
 template <typename R, int CT, int NR, bool NARROW>
@@ -1088,7 +1089,7 @@ __device__ __forceinline__ void generalValues(SFParams const& P,
                 for (int q = 0; q < S; ++q) acc[a * S + q] += v * phi[q];
             }
     });
-    flushCells<R, kPairGenRuns * S>(w, acc, u.cell, nr * S);
+    flushCells<R, kPairGenRuns * S>(w, acc, u.cell, pairUnitCells(u));
 }
 
 template <typename R, bool NARROW>
@@ -1138,7 +1139,7 @@ __device__ __forceinline__ void compactValues(SFParams const& P,
                 for (int s = 0; s < S; ++s) acc[a * S + s] += v * phi[s];
             }
     });
-    flushCells<R, N>(w, acc, u.cell, nr * S);
+    flushCells<R, N>(w, acc, u.cell, pairUnitCells(u));
 }
 
 template <typename R, int CT, int NZ, int MASK, bool NARROW>

@@ -66,6 +66,22 @@ struct PairUnit
     double   zeta[4];     // ladder
 };
 
+// Cells of a unit.  PK_POW2 units have those of PairParams::slots values of
+// zeta, which may be fewer than the slots a kernel is compiled for: kernels
+// touch these cells and no others.
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+inline int pairUnitCells(PairUnit const& u)
+{
+    switch (u.kind)
+    {
+    case PK_GENERAL: return u.nr * kPairGenShapes;
+    case PK_COMPACT: return u.nr * kPairCompShapes;
+    default: return 2 * u.nr * u.ns;
+    }
+}
+
 struct PairRun
 {
     double eta, rs;                       // exponential; compact: (rl, rc)

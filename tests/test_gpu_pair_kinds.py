@@ -1,0 +1,58 @@
+"""Two-pass symmetry-function kernels on potentials that no committed one
+stands for, against the kernels that form dG/dr: symmetry functions of h2o_52
+replaced, random networks.  Tolerances as in test_gpu_pair_path.py."""
+import os
+
+import numpy as np
+import pytest
+
+from test_gpu_pair_path import GOLD, _cluster, _compare, gpu  # noqa: F401
+
+pytestmark = pytest.mark.gpu
+
+BASE = os.path.join(GOLD, "potentials/h2o_52")
+PAIRS = (("H", "H"), ("H", "O"), ("O", "O"))
+
+
+def _write(out, functions, cutoff="1 0.0"):
+    """A potential directory: `functions` ("type neighbors parameters") for
+    both elements, networks with weights of a fixed seed."""
+    with open(os.path.join(BASE, "input.nn")) as fh:
+        keep = [x for x in fh if x.split()[:1] not in (["symfunction_short"],
+                                                       ["cutoff_type"])]
+    with open(os.path.join(out, "input.nn"), "w") as fh:
+        fh.writelines(keep)
+        fh.write(f"cutoff_type {cutoff}\n")
+        fh.writelines(f"symfunction_short {c} {s}\n" for c in "HO"
+                      for s in functions)
+    per = len(functions)
+    with open(os.path.join(out, "scaling.data"), "w") as fh:
+        for e in (1, 2):
+            for k in range(per):
+                fh.write(f"{e} {k + 1} 0.0 10.0 1.0 1.0\n")
+    widths = [per, 25, 25, 1]
+    count = sum(i * o + o for i, o in zip(widths[:-1], widths[1:]))
+    rng = np.random.default_rng(4)
+    for z in (1, 8):
+        with open(os.path.join(out, f"weights.{z:03d}.data"), "w") as fh:
+            fh.writelines(f"{v:.16e}\n"
+                          for v in rng.uniform(-0.3, 0.3, count))
+    return str(out)
+
+
+def _pow2(pairs, zetas, runs, rc=12.0):
+    return [f"3 {a} {b} {0.01 * (r + 1)} {lam} {z} {rc}" for a, b in pairs
+            for r in range(runs) for z in zetas for lam in ("-1", "1")]
+
+
+@pytest.mark.parametrize("n", [3, 33, 97])
+@pytest.mark.parametrize("other", ["3 H H 0.02 1.0 3.0 12.0",
+                                   "3 H H 0.02 1.0 2.5 12.0",
+                                   "3 H H 0.02 1.0 1.0 12.0 1.5"])
+def test_few_cells_behind_powers_of_two(gpu, monkeypatch, tmp_path, other, n):
+    """Powers of two up to 4 in a kernel with slots up to 16, one radial
+    function per neighbor element behind the last unit."""
+    sf = ["2 H 0.02 0.0 12.0", "2 O 0.05 0.0 12.0", other]
+    d = _write(tmp_path, sf + _pow2(PAIRS[1:], (1, 4), 4))
+    pos, elem = _cluster(n, 2, n, 3.0)
+    _compare(d, pos, elem, None, monkeypatch)
