@@ -2240,30 +2240,61 @@ struct n2p2b_context
         if (E > 0x7ffffffeL || targets > 0x7ffffffeL)
             throw std::invalid_argument("ERROR: Neighbor list too large.\n");
         activate();
+        // The entries are checked on the device before any state changes.
+        engRaw.ensure(36 * (std::size_t)std::max(E, 1L));
+        engScratch.ensure(sizeof(int) * (std::size_t)(targets + 1 + E));
+        EngineListLaunch G;
+        G.n = num;
+        G.entries = E;
+        G.numElements = ne;
+        G.numTargets = targets;
+        // Raw entries: displacements, indices, elements.
+        unsigned char* const raw = engRaw.as<unsigned char>();
+        G.rawDr = reinterpret_cast<double const*>(raw);
+        G.rawIndex = reinterpret_cast<int64_t const*>(raw + 24 * E);
+        G.rawElem = reinterpret_cast<int const*>(raw + 32 * E);
+        // The counts first: the scan reads them as 16-byte vectors.
+        G.revCount = engScratch.as<int>();
+        G.revTmp = engScratch.as<int>() + targets;
+        G.bad = engScratch.as<int>() + targets + E;
+        engUp.copy(device, stream,
+                   {{raw, drIn, 24 * (std::size_t)E},
+                    {raw + 24 * E, index, 8 * (std::size_t)E},
+                    {raw + 32 * E, nelems, 4 * (std::size_t)E}});
+        launchEngineCheck(G, stream);
+        checkLaunch("neighbor list check");
+        std::vector<int> byElem, off(num + 1, 0);
+        byElem.reserve(num);
+        ElemStarts starts{};
+        for (int e = 0; e < ne; ++e)
+        {
+            starts.start[e] = (int)byElem.size();
+            for (long i = 0; i < num; ++i)
+                if (elems[i] == e) byElem.push_back((int)i);
+        }
+        for (int e = ne; e <= kMaxElem; ++e)
+            starts.start[e] = (int)byElem.size();
+        int maxCnt = 0;
+        for (long i = 0; i < num; ++i)
+        {
+            off[i + 1] = off[i] + (int)counts[i];
+            maxCnt = std::max(maxCnt, (int)counts[i]);
+        }
+        int bad = 0;
+        ck(cudaMemcpyAsync(&bad, G.bad, sizeof(int), cudaMemcpyDeviceToHost,
+                           stream), "read neighbor list check");
+        ck(cudaStreamSynchronize(stream), "neighbor list check");
+        if (bad)
+            throw std::invalid_argument("ERROR: Bad neighbor entry.\n");
+
+        invalidate();
         n = num;
         numStructs = 0;
         externalNL = true;
         numTargets = targets;
         graphValid = false;
         elemHost.assign(elems, elems + num);
-        std::vector<int> byElem;
-        byElem.reserve(n);
-        std::memset(&es, 0, sizeof(es));
-        for (int e = 0; e < ne; ++e)
-        {
-            es.start[e] = (int)byElem.size();
-            for (long i = 0; i < n; ++i)
-                if (elemHost[i] == e) byElem.push_back((int)i);
-        }
-        es.start[ne] = (int)byElem.size();
-        for (int e = ne + 1; e <= kMaxElem; ++e) es.start[e] = es.start[ne];
-        std::vector<int> off(n + 1, 0);
-        int maxCnt = 0;
-        for (long i = 0; i < n; ++i)
-        {
-            off[i + 1] = off[i] + (int)counts[i];
-            maxCnt = std::max(maxCnt, (int)counts[i]);
-        }
+        es = starts;
         ensureStructureBuffers();
         capacity = std::max(capacity, std::max(E, 1L));
         ensureEntryBuffers();
@@ -2272,21 +2303,8 @@ struct n2p2b_context
         revOff.ensure(sizeof(int) * (targets + 1));
         revEntry.ensure(sizeof(int) * std::max(E, 1L));
         Ftarget.ensure(sizeof(double) * 3 * targets);
-        engRaw.ensure(36 * (std::size_t)std::max(E, 1L));
-        engScratch.ensure(sizeof(int) * (std::size_t)(targets + 1 + E));
-        invalidate();
-        EngineListLaunch G;
-        G.n = n;
-        G.entries = E;
-        G.numElements = ne;
-        G.numTargets = targets;
         G.scale = pot.normalize ? pot.convLength : 1.0;
         G.off = nbrOff.as<int>();
-        // Raw entries: displacements, indices, elements.
-        unsigned char* const raw = engRaw.as<unsigned char>();
-        G.rawDr = reinterpret_cast<double const*>(raw);
-        G.rawIndex = reinterpret_cast<int64_t const*>(raw + 24 * E);
-        G.rawElem = reinterpret_cast<int const*>(raw + 32 * E);
         G.nbrCountElem = nbrCountElem.as<int>();
         G.nbrIdx = nbrIdx.as<int>();
         G.nbrEl = nbrEl.as<int8_t>();
@@ -2294,16 +2312,8 @@ struct n2p2b_context
         G.dy = dy.as<double>();
         G.dz = dz.as<double>();
         G.dd = dd.as<double>();
-        // The counts first: the scan reads them as 16-byte vectors.
-        G.revCount = engScratch.as<int>();
-        G.revTmp = engScratch.as<int>() + targets;
-        G.bad = engScratch.as<int>() + targets + E;
         G.revOff = revOff.as<int>();
         G.revEntry = revEntry.as<int>();
-        engUp.copy(device, stream,
-                   {{raw, drIn, 24 * (std::size_t)E},
-                    {raw + 24 * E, index, 8 * (std::size_t)E},
-                    {raw + 32 * E, nelems, 4 * (std::size_t)E}});
         auto up = [&](DevBuf& b, void const* h, std::size_t bytes) {
             if (bytes)
                 ck(cudaMemcpyAsync(b.p, h, bytes, cudaMemcpyHostToDevice,
@@ -2314,13 +2324,7 @@ struct n2p2b_context
         up(nbrOff, off.data(), sizeof(int) * (n + 1));
         launchEngineList(G, stream);
         checkLaunch("neighbor list kernels");
-        int bad = 0;
-        ck(cudaMemcpyAsync(&bad, G.bad, sizeof(int), cudaMemcpyDeviceToHost,
-                           stream), "read neighbor list check");
         ck(cudaStreamSynchronize(stream), "neighbor list upload");
-        if (bad)
-            throw std::invalid_argument("ERROR: Bad neighbor entry.\n");
-        invalidate();
         haveNL = true;
         lastMaxNbr = maxCnt;
         sfCap = 0;

@@ -82,6 +82,8 @@ struct EngineListLaunch
     int*           bad = nullptr;      // set if an entry is out of range
 };
 
+// Looks the raw entries over (sets *bad); the list from entries that passed.
+void launchEngineCheck(EngineListLaunch const& L, cudaStream_t s);
 void launchEngineList(EngineListLaunch const& L, cudaStream_t s);
 // off[0 .. n] = exclusive prefix sums of cnt[0 .. n); both 16-byte aligned.
 void launchOffsetScan(long n, int const* cnt, int* off, cudaStream_t s);

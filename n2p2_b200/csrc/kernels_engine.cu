@@ -11,6 +11,19 @@ namespace n2p2b
 namespace
 {
 
+// Thread per entry: elements and targets are in range.  It runs before
+// anything of the list that is in place is overwritten, so that a refused
+// list leaves the previous one (or the structure) as it was.
+__global__ void engineCheckKernel(EngineListLaunch const L)
+{
+    long const e = (long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= L.entries) return;
+    int const el = L.rawElem[e];
+    int64_t const idx = L.rawIndex[e];
+    if (el < 0 || el >= L.numElements || idx < 0 || idx >= L.numTargets)
+        *L.bad = 1;
+}
+
 // Warp per atom: stable regrouping of its entries by neighbor element.  The
 // distance is formed as InterfaceLammps::addNeighbor does (n.d = sqrt(d2),
 // then scaled like the components), without contraction.  Entries are 36
@@ -28,30 +41,13 @@ engineGroupKernel(EngineListLaunch const L)
     int at[kMaxElem];
 #pragma unroll
     for (int e = 0; e < kMaxElem; ++e) at[e] = 0;
-    bool bad = false;
     for (int t = lane; t - lane < cnt; t += 32)
     {
-        int el = -1;
-        if (t < cnt)
-        {
-            el = L.rawElem[b + t];
-            int64_t const idx = L.rawIndex[b + t];
-            if (el < 0 || el >= L.numElements || idx < 0
-                || idx >= L.numTargets)
-            {
-                bad = true;
-                el = -1;
-            }
-        }
+        int const el = t < cnt ? L.rawElem[b + t] : -1;
 #pragma unroll
         for (int e = 0; e < kMaxElem; ++e)
             if (e < L.numElements)
                 at[e] += __popc(__ballot_sync(0xffffffffu, el == e));
-    }
-    if (__any_sync(0xffffffffu, bad))
-    {
-        if (lane == 0) *L.bad = 1;
-        return;
     }
     int run = 0;
 #pragma unroll
@@ -98,7 +94,6 @@ engineGroupKernel(EngineListLaunch const L)
 // segment is that of the atomics; engineSortKernel makes it ascending.
 __global__ void engineFillKernel(EngineListLaunch const L)
 {
-    if (*L.bad) return;
     long const e = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= L.entries) return;
     int const m = L.nbrIdx[e];
@@ -111,7 +106,6 @@ __global__ void engineFillKernel(EngineListLaunch const L)
 __global__ void __launch_bounds__(128)
 engineSortKernel(EngineListLaunch const L)
 {
-    if (*L.bad) return;
     int const lane = threadIdx.x & 31;
     long const m = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (m >= L.numTargets) return;
@@ -128,10 +122,17 @@ engineSortKernel(EngineListLaunch const L)
 
 } // namespace
 
+void launchEngineCheck(EngineListLaunch const& L, cudaStream_t s)
+{
+    cudaMemsetAsync(L.bad, 0, sizeof(int), s);
+    if (L.entries == 0) return;
+    noteLaunches(1);
+    engineCheckKernel<<<(unsigned)((L.entries + 255) / 256), 256, 0, s>>>(L);
+}
+
 void launchEngineList(EngineListLaunch const& L, cudaStream_t s)
 {
     int const tb = 128, warps = tb / 32;
-    cudaMemsetAsync(L.bad, 0, sizeof(int), s);
     cudaMemsetAsync(L.revCount, 0, sizeof(int) * (std::size_t)L.numTargets, s);
     noteLaunches(L.entries > 0 ? 4 : 2);
     engineGroupKernel<<<(unsigned)((L.n + warps - 1) / warps), tb, 0, s>>>(L);
