@@ -28,6 +28,18 @@
 // for the whole warp, and add the four slices at the end.  Each pair term
 // has one writer: no atomics, fixed order.
 //
+// Precision.  The FP32 kernels form a triplet's terms in FP32, the sums over
+// its members among them, and add them up in FP64: over an owner's partners,
+// the radial functions of a neighbor, the units, the lanes and the neighbors.
+// The storing kernels add a member's partners in FP32 and the members in
+// FP64.  Forces' rms error against FP64 with exact dE/dG, 12 water boxes of
+// 192 to 720 atoms, two passes / storing kernels: 52 functions 1.47e-7 /
+// 2.32e-7, 92 functions 2.77e-7 / 5.03e-7, tanh^3 cutoff (27 and 30
+// functions) 2.45e-7 / 2.47e-7; with FP32 sums over partners and radial
+// functions 1.52, 3.07 and 2.61e-7.  FP64 inside the triplet as well leaves
+// the errors where they are (92 functions 2.94e-7 against 3.08e-7 with FP32
+// sums, 256 molecules) and takes a third more time.
+//
 // Bounds.  Memory is small (the neighbor entries once per pass, 24 B written
 // per entry); the FP64 instructions (about 80 a triplet for the values, 130
 // per owner for the forces, 3 runs x 4 shapes) and their latency at 12 to 16
@@ -540,7 +552,8 @@ __device__ __forceinline__ void stageAtom(SFParams const& P,
             break;
         }
         double const d = L.dd[h.beg + e];
-        R const r = R(d), ir = R(1.0 / d);
+        double const id = 1.0 / d;
+        R const r = R(d), ir = R(id);
         R const x = R(L.dx[h.beg + e]), y = R(L.dy[h.beg + e]),
                 z = R(L.dz[h.beg + e]);
         int el = 0;
@@ -588,7 +601,8 @@ __device__ __forceinline__ void stageAtom(SFParams const& P,
             if (DERIV) S.rad[(2 * f + 1) * cs + t] = dv * ir;
         }
         if (!DERIV) continue;
-        R al = R(0), fc = R(0), dfc = R(0), ZZ = R(1);
+        double al = 0.0;
+        R fc = R(0), dfc = R(0), ZZ = R(1);
         int last = -1;
         for (int q = T.radialBeg[ec]; q < T.radialBeg[ec + 1]; ++q)
         {
@@ -617,9 +631,9 @@ __device__ __forceinline__ void stageAtom(SFParams const& P,
             }
             R v, dv;
             radialFdf<R>(P, pr, r, fc, dfc, S.tab, v, dv);
-            al += (C[pr.cell] * ZZ) * dv;
+            al += (double)((C[pr.cell] * ZZ) * dv);
         }
-        arad[t] = al * ir;
+        arad[t] = R(al * id);
     }
 }
 
@@ -1363,13 +1377,13 @@ pairValueKernel(__grid_constant__ SFParams const P,
 // Forces pass.
 // ---------------------------------------------------------------------------
 
-// Owner j's values and its sums: al along dr_ij and the vector (vx, vy, vz)
+// Owner j's values and its sums (FP64 in all forms): al along dr_ij and the vector (vx, vy, vz)
 // of the coefficients along dr_ik times dr_ik.
 template <typename R>
 struct Owner
 {
-    R x, y, z, ir, r2;
-    R al, vx, vy, vz;
+    R      x, y, z, ir, r2;
+    double al, vx, vy, vz;
 };
 
 // One lane's share of an owner's partners in a unit: entries at, at + kSl,
@@ -1407,7 +1421,7 @@ __device__ __forceinline__ void pow2Forces(SFParams const& P,
     int const slot = u.fcSlot, none = W.cs - 1;
     R const of = fcOf(W, slot, p.t), odf = W.dfc[slot * W.cs + p.t];
     unsigned const mask = MASK ? (unsigned)MASK : u.mask;
-    R al = R(0), vx = R(0), vy = R(0), vz = R(0);
+    double al = 0.0, vx = 0.0, vy = 0.0, vz = 0.0;
     P2 const* const C2 = reinterpret_cast<P2 const*>(C);
     R h1[NR];             // zeta = 1: d/dcos is a constant
 #pragma unroll
@@ -1496,10 +1510,10 @@ __device__ __forceinline__ void pow2Forces(SFParams const& P,
             a1 += x3;
             ga -= x3;
         }
-        al += a1;
-        vx += ga * B.x;
-        vy += ga * B.y;
-        vz += ga * B.z;
+        al += (double)a1;
+        vx += (double)(ga * B.x);
+        vy += (double)(ga * B.y);
+        vz += (double)(ga * B.z);
     }
     o.al = al;
     o.vx = vx;
@@ -1533,7 +1547,7 @@ __device__ __forceinline__ void ladderForces(SFParams const& P,
         prog[z] = u.prog[z];
         zeta[z] = R(u.zeta[z]);
     }
-    R al = R(0), vx = R(0), vy = R(0), vz = R(0);
+    double al = 0.0, vx = 0.0, vy = 0.0, vz = 0.0;
     P2 const* const C2 = reinterpret_cast<P2 const*>(C);
 #pragma unroll 1
     for (int st = 0; st < p.steps; ++st)
@@ -1597,10 +1611,10 @@ __device__ __forceinline__ void ladderForces(SFParams const& P,
             a1 += x3;
             ga -= x3;
         }
-        al += a1;
-        vx += ga * B.x;
-        vy += ga * B.y;
-        vz += ga * B.z;
+        al += (double)a1;
+        vx += (double)(ga * B.x);
+        vy += (double)(ga * B.y);
+        vz += (double)(ga * B.z);
     }
     o.al = al;
     o.vx = vx;
@@ -1624,7 +1638,7 @@ __device__ __forceinline__ void generalForces(SFParams const& P,
     PairRun const* const runs = tb.r + u.run;
     PairShape const* const sh = tb.s + u.shape;
     P2 const* const C2 = reinterpret_cast<P2 const*>(C);
-    R al = R(0), vx = R(0), vy = R(0), vz = R(0);
+    double al = 0.0, vx = 0.0, vy = 0.0, vz = 0.0;
 #pragma unroll 1
     for (int st = 0; st < p.steps; ++st)
     {
@@ -1686,10 +1700,10 @@ __device__ __forceinline__ void generalForces(SFParams const& P,
             a1 += x3;
             ga -= x3;
         }
-        al += a1;
-        vx += ga * B.x;
-        vy += ga * B.y;
-        vz += ga * B.z;
+        al += (double)a1;
+        vx += (double)(ga * B.x);
+        vy += (double)(ga * B.y);
+        vz += (double)(ga * B.z);
     }
     o.al = al;
     o.vx = vx;
@@ -1710,7 +1724,7 @@ __device__ __forceinline__ void compactForces(SFParams const& P,
     PairRun const* const runs = tb.r + u.run;
     PairShape const* const sh = tb.s + u.shape;
     P2 const* const C2 = reinterpret_cast<P2 const*>(C);
-    R al = R(0), vx = R(0), vy = R(0), vz = R(0);
+    double al = 0.0, vx = 0.0, vy = 0.0, vz = 0.0;
 #pragma unroll 1
     for (int st = 0; st < p.steps; ++st)
     {
@@ -1770,10 +1784,10 @@ __device__ __forceinline__ void compactForces(SFParams const& P,
         x3 *= ir3;
         R const mh = (x2 * dacos) * ir;
         R const ga = mh - x3;
-        al += x1 - (mh * dot) * (o.ir * o.ir) + x3;
-        vx += ga * B.x;
-        vy += ga * B.y;
-        vz += ga * B.z;
+        al += (double)(x1 - (mh * dot) * (o.ir * o.ir) + x3);
+        vx += (double)(ga * B.x);
+        vy += (double)(ga * B.y);
+        vz += (double)(ga * B.z);
     }
     o.al = al;
     o.vx = vx;
@@ -1880,7 +1894,7 @@ pairTermKernel(__grid_constant__ SFParams const P,
             for (int k = tm.tid; k < nc; k += Tm::kThreads)
             {
                 PairCell const ce = tb.c[c0 + k];
-                C[k] = ce.sf >= 0 ? row[ce.sf] * R(ce.fn) : R(0);
+                C[k] = ce.sf >= 0 ? R((double)row[ce.sf] * ce.fn) : R(0);
             }
         }
         Tm::sync();
@@ -2069,10 +2083,10 @@ pairTermKernel(__grid_constant__ SFParams const P,
                     if (u.narrow) compactForces<R, true>(P, tb, u, Cu, W, p, o);
                     else compactForces<R, false>(P, tb, u, Cu, W, p, o);
                 }
-                Al += (double)o.al;
-                Vx += (double)o.vx;
-                Vy += (double)o.vy;
-                Vz += (double)o.vz;
+                Al += o.al;
+                Vx += o.vx;
+                Vy += o.vy;
+                Vz += o.vz;
             }
     #pragma unroll
             for (int d = 1; d < kSl; d <<= 1)
