@@ -16,6 +16,21 @@ bool isRadial(int type)
     return type == 2 || type == 12 || type == 20 || type == 23;
 }
 
+// The exponentials take any exponent from 0 down whose size in their unit
+// (ln 2 / 256) stays below 2^31; eta < 0 is left to the other kernels.  The
+// largest sums of squares are those with the record of a partner far away:
+// neighbors up to `rc` (the potential's largest cutoff) from the atom, the
+// record at 2 rc, 3 rc between the two.
+bool exponentFits(double eta, double rs, double rc, bool radial)
+{
+    auto square = [](double x) { return x * x; };
+    double const a = std::fabs(rs);
+    double const sum = radial ? square(rc + a)
+        : square(std::max(rc, a)) + square(std::max(2.0 * rc, a))
+          + square(std::max(3.0 * rc, a));
+    return eta >= 0.0 && eta * sum < 5.8e6;
+}
+
 // Index of (group's rc, weighted) among the element's staged cutoff values,
 // added if new; -1 if there are too many.
 int fcSlotOf(SFParams const& P, PairTables& t, int beg, int group, int weighted)
@@ -139,9 +154,9 @@ bool addGroup(SFParams const& P, PairTables& t, int fcBeg, int radBeg, int gi,
             t.why = "an angular function with lambda or zeta 0";
             return false;
         }
-        if (!(M[m].eta * g.rc2 < 1e6))
+        if (!exponentFits(M[m].eta, M[m].rs, 0.5 * t.p.farAway, false))
         {
-            t.why = "a very large eta";
+            t.why = "a negative or very large eta";
             return false;
         }
         if (M[m].rs < 0.0)
@@ -401,9 +416,9 @@ void buildPairTables(SFParams const& P, PairTables& t)
                     r.center = mm.factorDeriv;
                     r.scale = mm.zetaLambda;
                 }
-                else if (!(mm.eta * d.rc2 < 1e6))
+                else if (!exponentFits(mm.eta, mm.rs, rcMax, true))
                 {
-                    t.why = "a very large eta";
+                    t.why = "a negative or very large eta";
                     return;
                 }
                 t.radials.push_back(r);

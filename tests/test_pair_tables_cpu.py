@@ -80,3 +80,24 @@ def test_cells_of_units(tables, zetas, runs, radials, other):
                 at += 1
             else:
                 assert int(line[2]) == at
+
+
+@pytest.mark.parametrize("zeta", [1.0, 3.0, 2.5])
+@pytest.mark.parametrize("radial,eta,rs,served", [
+    (r, eta, rs, ok) for r in (True, False) for eta, rs, ok in (
+        (0.0, 0.0, True), (4.0, 0.0, True), (4.0, 1.5, True),
+        (100.0, 8.0, True), (-1e-4, 0.0, False), (-0.6, 0.0, False),
+        (-0.6, 2.0, False), (5.0, 1100.0, False), (50000.0, 0.0, False))
+] + [(False, 2870.0, 0.0, True), (False, 2885.0, 0.0, False),
+     (True, 40200.0, 0.0, True), (True, 40400.0, 0.0, False)])
+def test_exponents(tables, zeta, radial, eta, rs, served):
+    """-eta (sum of squares) has to stay between 0 and -5.8e6 (2^31 ln 2 /
+    256) for every partner that the kernels form it for, the far one of idle
+    lanes included (14 rc^2; radial: rc^2); other potentials are left to the
+    storing kernels.  The function's own cutoff (6) is not the largest (12)."""
+    member, plain = (eta, rs, 1.0, zeta), (0.01, 0.0, 1.0, zeta)
+    groups = [(0, 3, 0, 0, 6.0, [plain if radial else member]),
+              (0, 2, 0, -1, 6.0, [member if radial else plain]),
+              (0, 2, 0, -1, 12.0, [(0.01, 0.0, 0.0, 0.0)])]
+    out = tables(1, groups)
+    assert (out[0][0] == "ok") == served
