@@ -238,7 +238,9 @@ int n2p2b_launch_graph(n2p2b_context* ctx);
 
 /* Autotuner: times every launch configuration (symmetry-function kernel
  * variant and work ordering, neighbor-list warps per block for batches) on
- * the current structure(s), keeps the fastest for their size bucket
+ * the current structure(s) -- where the two-pass path evaluates, the variants
+ * are those of the kernels that form dG/dr and are timed if the context has
+ * used them --, keeps the fastest for their size bucket
  * (log2 atoms per structure, per precision) and applies it to later
  * structures of that bucket.  `report` receives the choice. */
 int n2p2b_autotune(n2p2b_context* ctx, int use_forces, int repetitions,

@@ -2461,7 +2461,8 @@ struct n2p2b_context
         checkLaunch("kernel launch");
     }
 
-    int finishStatus()
+    // Waits for what was enqueued and throws if its kernels gave up.
+    void checkStatus()
     {
         int const flags = readStatus();
         if (flags & (FLAG_NBR_OVERFLOW | FLAG_SF_CAPACITY))
@@ -2477,6 +2478,11 @@ struct n2p2b_context
         if (flags & FLAG_SF_PATH)
             throw std::runtime_error("ERROR: Internal: symmetry-function "
                                      "kernel without a needed path.\n");
+    }
+
+    int finishStatus()
+    {
+        checkStatus();
         haveNL = haveSF = haveNN = haveE = true;
         if (ewCheck) accountEW();
         return 0;
@@ -2590,22 +2596,26 @@ struct n2p2b_context
         cudaEvent_t a, b;
         ck(cudaEventCreate(&a), "event");
         ck(cudaEventCreate(&b), "event");
-        auto timeIt = [&]() {
+        auto timeIt = [&](auto&& enqueue, auto&& finish) {
             sfGrid = 0;
-            enqueueAll(forces);                 // warm
-            finishStatus();
+            enqueue();                          // warm
+            finish();
             double best = 1e30;
             for (int r = 0; r < reps; ++r)
             {
                 ck(cudaEventRecord(a, stream), "record");
-                enqueueAll(forces);
+                enqueue();
                 ck(cudaEventRecord(b, stream), "record");
-                finishStatus();
+                finish();
                 float ms = 0.0f;
                 ck(cudaEventElapsedTime(&ms, a, b), "elapsed");
                 best = std::min(best, (double)ms);
             }
             return best;
+        };
+        auto evaluation = [&] {
+            return timeIt([&] { enqueueAll(forces); },
+                          [&] { finishStatus(); });
         };
         if (sfVariant < 0)
         {
@@ -2613,26 +2623,59 @@ struct n2p2b_context
             sfSortCats = sfDefaultSort(sfp);
         }
         TuneChoice const start{sfVariant, sfSortCats, nlWarpsPerBlock, 0.0};
-        double const t0 = timeIt();
+        double const t0 = evaluation();
         TuneChoice best{sfVariant, sfSortCats, nlWarpsPerBlock, t0};
         std::string rep;
-        // The two-pass path has no variants: only the neighbor list's
-        // launch is left to choose.
-        bool const pair = pairUsable();
-        for (int v = 0; v < kSFVariants; ++v)
-            for (int so : {1, 3, 5, 7})
+        // Variants and item orders of the storing kernels (the staged ones
+        // ignore the order).
+        auto variants = [&](auto&& visit) {
+            for (int v = 0; v < kSFVariants; ++v)
+                for (int so : {1, 3, 5, 7})
+                    if (v < 6 || so == 5) visit(v, so);
+        };
+        if (!pairUsable())
+            variants([&](int v, int so) {
                 for (int w : nls)
                 {
-                    if (pair && (v != start.variant || so != start.sortCats))
-                        continue;
-                    // The staged kernel ignores the item order.
-                    if (v >= 6 && so != 5) continue;
                     sfVariant = v;
                     sfSortCats = so;
                     nlWarpsPerBlock = w;
-                    double const t = timeIt();
+                    double const t = evaluation();
                     if (t < best.ms) best = TuneChoice{v, so, w, t};
                 }
+            });
+        else
+        {
+            // The two-pass path has no variants: an evaluation leaves the
+            // neighbor list's launch to choose.
+            for (int w : nls)
+            {
+                nlWarpsPerBlock = w;
+                double const t = evaluation();
+                if (t < best.ms) best.nlWarps = w, best.ms = t;
+            }
+            // Contexts that use dG/dr (training, single steps) have its
+            // buffer: their storing kernel is timed alone.
+            if (forces && dGdr.p)
+            {
+                Gother.ensure(realBytes() * n * maxSF);
+                auto storing = [&] {
+                    return timeIt([&] { enqueueStoredSF(true, Gother.p); },
+                                  [&] { checkStatus(); });
+                };
+                double least = storing();
+                variants([&](int v, int so) {
+                    sfVariant = v;
+                    sfSortCats = so;
+                    double const t = storing();
+                    if (t >= least) return;
+                    least = t;
+                    best.variant = v;
+                    best.sortCats = so;
+                });
+                haveDGdr = false;
+            }
+        }
         cudaEventDestroy(a);
         cudaEventDestroy(b);
         sfVariant = best.variant;
