@@ -1451,7 +1451,7 @@ struct n2p2b_context
         Gother.ensure(realBytes() * n * maxSF);
         enqueueStoredSF(true, Gother.p);
         checkLaunch("symmetry-function derivatives");
-        ck(cudaStreamSynchronize(stream), "synchronize");
+        checkStatus();
         haveDGdr = true;
     }
 
