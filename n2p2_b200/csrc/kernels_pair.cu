@@ -204,10 +204,14 @@ void launchPair(int pass, SFParams const& P, PairParams const& host,
         L.wpa = kWarpsPerCta;
         shm = layout(host, L, pass);
     }
-    // N2P2B_PAIR_WPA=1 or 4 asks for one of the two (measurements, tests).
+    // N2P2B_PAIR_WPA=1 or 4 asks for one of the two (measurements, tests); one
+    // warp per atom only where four atoms' shared memory fits a block.
     if (char const* e = std::getenv("N2P2B_PAIR_WPA"))
     {
-        L.wpa = std::atoi(e) == 1 ? 1 : kWarpsPerCta;
+        L.wpa = 1;
+        if (std::atoi(e) != 1
+            || layout(host, L, pass) > (std::size_t)kPairSmemBlock)
+            L.wpa = kWarpsPerCta;
         shm = layout(host, L, pass);
     }
     noteLaunches(1);

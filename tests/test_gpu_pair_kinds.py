@@ -6,7 +6,9 @@ import os
 import numpy as np
 import pytest
 
-from test_gpu_pair_path import GOLD, _cluster, _compare, gpu  # noqa: F401
+from n2p2_b200 import synth
+from test_gpu_pair_path import (GOLD, _cluster, _compare,  # noqa: F401
+                                _prediction, gpu)
 
 pytestmark = pytest.mark.gpu
 
@@ -56,3 +58,24 @@ def test_few_cells_behind_powers_of_two(gpu, monkeypatch, tmp_path, other, n):
     d = _write(tmp_path, sf + _pow2(PAIRS[1:], (1, 4), 4))
     pos, elem = _cluster(n, 2, n, 3.0)
     _compare(d, pos, elem, None, monkeypatch)
+
+
+def test_one_warp_per_atom_asked_for(gpu, monkeypatch):
+    """327 neighbors and weighted functions: in the forces pass four atoms do
+    not fit a block, so asking for one warp per atom is not followed there
+    (the values pass follows: sums in another order)."""
+    box, pos, elem = synth.water_box(64, 9)
+    out = []
+    for wpa in (None, "1"):
+        if wpa:
+            monkeypatch.setenv("N2P2B_PAIR_WPA", wpa)
+        else:
+            monkeypatch.delenv("N2P2B_PAIR_WPA", raising=False)
+        p = _prediction(os.path.join(GOLD, "potentials/h2o_wtd"), False,
+                        monkeypatch)
+        e, f = p.predict(0.7 * pos, elem, 0.7 * box)
+        assert p.neighbor_counts().max() > 300
+        out.append((e, f))
+    (e0, f0), (e1, f1) = out
+    assert abs(e1 - e0) <= 1e-10 * abs(e0)
+    assert np.abs(f1 - f0).max() <= 1e-10 * np.abs(f0).max()
