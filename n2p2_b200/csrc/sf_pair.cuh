@@ -33,9 +33,9 @@
 // the radial functions of a neighbor, the units, the lanes and the neighbors.
 // The storing kernels add a member's partners in FP32 and the members in
 // FP64.  Forces' rms error against FP64 with exact dE/dG, 12 water boxes of
-// 192 to 720 atoms, two passes / storing kernels: 52 functions 1.47e-7 /
-// 2.32e-7, 92 functions 2.77e-7 / 5.03e-7, tanh^3 cutoff (27 and 30
-// functions) 2.45e-7 / 2.47e-7; with FP32 sums over partners and radial
+// 192 to 720 atoms, two passes / storing kernels: 52 functions 1.50e-7 /
+// 2.32e-7, 92 functions 2.79e-7 / 5.03e-7, tanh^3 cutoff (27 and 30
+// functions) 2.51e-7 / 2.47e-7; with FP32 sums over partners and radial
 // functions 1.52, 3.07 and 2.61e-7.  FP64 inside the triplet as well leaves
 // the errors where they are (92 functions 2.94e-7 against 3.08e-7 with FP32
 // sums, 256 molecules) and takes a third more time.
@@ -208,16 +208,19 @@ static __device__ double const kPairExp2[kPairExpSize] = {
     0x1.fe9d96b2a23d9p+0,
 };
 
-// Constants of one run: eta in the exponential's unit.
+// Constants of one run: -eta in the exponential's unit, from the tables'
+// -eta / ln 2 and rounded once (in FP32 its error is the same for every
+// triplet of the run and does not average out).
 //   FP64: exp(-eta s) = 2^(k/256) 2^(f/256), k = rint(y), f = y - k with
 //   y = -eta s 256/ln2; f is formed by one fma from s (no product rounding),
 //   2^(f/256) - 1 by its Taylor polynomial of degree 4 in f (|f| <= 1/2:
 //   truncation below 4e-17), 2^(j/256) from the table.  The error is that of
 //   y's factor, |eta s| 2^-53, and 1 ulp, as for exp of the rounded
 //   product.  Results below 2^-1020 stay near 2^-1020.
-__device__ __forceinline__ double expScale(double eta)
+template <typename R>
+__device__ __forceinline__ R expScale(double e2)
 {
-    return eta * -0x1.71547652b82fep+8;
+    return sizeof(R) == 8 ? R(e2 * 256.0) : R(e2);
 }
 __device__ __forceinline__ double expScaled(double e2, double s,
                                             double const* tab)
@@ -233,10 +236,6 @@ __device__ __forceinline__ double expScaled(double e2, double s,
     double const tm = __hiloint2double(
         __double2hiint(tj) + ((k >> 8) << 20), __double2loint(tj));
     return fma(tm, q, tm);
-}
-__device__ __forceinline__ float expScale(float eta)
-{
-    return eta * -1.44269504f;
 }
 __device__ __forceinline__ float expScaled(float e2, float s, double const*)
 {
@@ -509,7 +508,7 @@ __device__ __forceinline__ void radialFdf(SFParams const& P,
         return;
     }
     R const d = r - R(m.rs), eta = R(m.eta);
-    R const e = expScaled(expScale(eta), d * d, tab);
+    R const e = expScaled(expScale<R>(m.center), d * d, tab);
     v = e * fc;
     dv = e * (dfc - R(2) * eta * d * fc);
 }
@@ -934,7 +933,7 @@ __device__ __forceinline__ void pow2Values(SFParams const& P,
     for (int c = 0; c < NZ * NR * 2; ++c) acc[c] = R(0);
     R e2[NR];
 #pragma unroll
-    for (int a = 0; a < NR; ++a) e2[a] = expScale(R(tb.r[u.run + a].eta));
+    for (int a = 0; a < NR; ++a) e2[a] = expScale<R>(tb.r[u.run + a].center);
     R const a2q = R(u.a2q), rc2 = R(u.rc2);
     bool const exact = u.exactMask != 0;
     int const slot = u.fcSlot;
@@ -996,7 +995,7 @@ __device__ __forceinline__ void ladderValues(SFParams const& P,
     R e2[NR];
 #pragma unroll
     for (int a = 0; a < NR; ++a)
-        e2[a] = expScale(R(tb.r[u.run + min(a, nr - 1)].eta));
+        e2[a] = expScale<R>(tb.r[u.run + min(a, nr - 1)].center);
     R const a2q = R(u.a2q), rc2 = R(u.rc2);
     bool const exact = u.exactMask != 0;
     int const slot = u.fcSlot, ns = u.ns;
@@ -1097,7 +1096,7 @@ __device__ __forceinline__ void generalValues(SFParams const& P,
                     x = (rA - rs) * (rA - rs) + (rB - rs) * (rB - rs);
                     if (NARROW) x += (r3 - rs) * (r3 - rs);
                 }
-                R const v = m * expScaled(expScale(R(runs[a].eta)), x,
+                R const v = m * expScaled(expScale<R>(runs[a].center), x,
                                           w.W.tab);
 #pragma unroll
                 for (int q = 0; q < S; ++q) acc[a * S + q] += v * phi[q];
@@ -1415,7 +1414,7 @@ __device__ __forceinline__ void pow2Forces(SFParams const& P,
     using P2 = typename V2<R>::T;
     R e2[NR];
 #pragma unroll
-    for (int a = 0; a < NR; ++a) e2[a] = expScale(R(tb.r[u.run + a].eta));
+    for (int a = 0; a < NR; ++a) e2[a] = expScale<R>(tb.r[u.run + a].center);
     R const a2q = R(u.a2q), qf = R(u.qf), rc2 = R(u.rc2);
     bool const exact = u.exactMask != 0;
     int const slot = u.fcSlot, none = W.cs - 1;
@@ -1534,7 +1533,7 @@ __device__ __forceinline__ void ladderForces(SFParams const& P,
     R e2[NR];
 #pragma unroll
     for (int a = 0; a < NR; ++a)
-        e2[a] = expScale(R(tb.r[u.run + min(a, nr - 1)].eta));
+        e2[a] = expScale<R>(tb.r[u.run + min(a, nr - 1)].center);
     R const a2q = R(u.a2q), qf = R(u.qf), rc2 = R(u.rc2);
     bool const exact = u.exactMask != 0;
     int const slot = u.fcSlot, ns = u.ns, none = W.cs - 1;
@@ -1671,7 +1670,7 @@ __device__ __forceinline__ void generalForces(SFParams const& P,
                 x = (rA - rs) * (rA - rs) + (rB - rs) * (rB - rs);
                 if (NARROW) x += (r3 - rs) * (r3 - rs);
             }
-            R const v = expScaled(expScale(eta), x, W.tab);
+            R const v = expScaled(expScale<R>(runs[a].center), x, W.tab);
             R b = R(0), h = R(0);
 #pragma unroll
             for (int j = 0; j < S / 2; ++j)

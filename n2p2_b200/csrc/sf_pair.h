@@ -85,7 +85,8 @@ inline int pairUnitCells(PairUnit const& u)
 struct PairRun
 {
     double eta, rs;                       // exponential; compact: (rl, rc)
-    double center, scale;                 // compact window function
+    double center, scale;                 // compact window function;
+                                          // exponential: center = -eta / ln 2
     int    core, asym;
     int    slot;                          // compact: staged radial values
     int    pad;
@@ -111,7 +112,7 @@ struct PairRadial
     int    cell;          // relative to the element's cells
     int    core, asym;
     double eta, rs;       // compact: rl, rc
-    double center, scale;
+    double center, scale; // exponential: center = -eta / ln 2
 };
 
 struct PairCell

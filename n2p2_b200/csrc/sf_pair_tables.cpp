@@ -11,6 +11,8 @@ namespace n2p2b
 namespace
 {
 
+constexpr double kMinusLog2E = -0x1.71547652b82fep+0;   // -1 / ln 2
+
 bool isRadial(int type)
 {
     return type == 2 || type == 12 || type == 20 || type == 23;
@@ -194,6 +196,7 @@ bool addGroup(SFParams const& P, PairTables& t, int fcBeg, int radBeg, int gi,
         PairRun r{};
         r.eta = m.eta;
         r.rs = m.rs;
+        r.center = m.eta * kMinusLog2E;
         if (compact)
         {
             r.center = m.factorDeriv;
@@ -409,6 +412,7 @@ void buildPairTables(SFParams const& P, PairTables& t)
                 r.cell = cells++;
                 r.eta = mm.eta;
                 r.rs = mm.rs;
+                r.center = mm.eta * kMinusLog2E;
                 if (r.compact)
                 {
                     r.core = mm.zetaInt;

@@ -79,3 +79,40 @@ def test_one_warp_per_atom_asked_for(gpu, monkeypatch):
     (e0, f0), (e1, f1) = out
     assert abs(e1 - e0) <= 1e-10 * abs(e0)
     assert np.abs(f1 - f0).max() <= 1e-10 * np.abs(f0).max()
+
+
+# Hard, exponential, polynomial and tanh cutoffs, the cosine with an inner
+# radius: the kernels of powers of two compiled for tanh^3 and polynomial 2
+# and for any cutoff, with slots up to 4 and up to 16.
+CUTOFFS = ["0", "2", "3", "4", "5", "6", "7", "8", "1 0.2", "6 0.3"]
+
+
+def _pow2_potential(out, cutoff, zetas):
+    sf = [f"2 {e} {eta} 0.0 12.0" for e in "HO" for eta in (0.01, 0.2, 1.0)]
+    out.mkdir()
+    return _write(out, sf + _pow2(PAIRS, zetas, 3), cutoff)
+
+
+@pytest.mark.parametrize("zetas", [(1, 2, 4), (1, 2, 4, 16)])
+@pytest.mark.parametrize("cutoff", CUTOFFS + ["1 0.0"])
+def test_powers_of_two_by_cutoff_mixed(gpu, monkeypatch, tmp_path, cutoff,
+                                       zetas):
+    """Errors against FP64 no larger than the storing kernels' by more than a
+    quarter (one box of 64 molecules; exact dE/dG)."""
+    from test_gpu_pair_mixed import _linear, _rms, _steps
+    monkeypatch.delenv("N2P2B_SF_VARIANT", raising=False)
+    src = _pow2_potential(tmp_path / "p", cutoff, zetas)
+    (tmp_path / "q").mkdir()
+    d = _linear(src, str(tmp_path / "q"))
+    exact = _prediction(d, False, monkeypatch)
+    mixed = _prediction(d, False, monkeypatch, "mixed")
+    box, pos, elem = synth.water_box(64, 8)
+    pos = pos + np.random.default_rng(1).normal(0.0, 0.1, pos.shape)
+    exact.predict(pos, elem, box)
+    want = exact.symmetry_functions(), exact.forces()
+    mixed.predict(pos, elem, box)
+    two = mixed.symmetry_functions(), mixed.forces()
+    for name, x, y, x0 in zip("GF", two, _steps(mixed), want):
+        e, s = _rms([x - x0]), _rms([y - x0])
+        print(f"{cutoff} {zetas}: {name} {e:.3e} / {s:.3e}")
+        assert 0.0 < e <= 1.25 * s
