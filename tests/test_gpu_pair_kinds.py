@@ -93,6 +93,15 @@ def _pow2_potential(out, cutoff, zetas):
     return _write(out, sf + _pow2(PAIRS, zetas, 3), cutoff)
 
 
+@pytest.mark.parametrize("n", [3, 33, 97])
+@pytest.mark.parametrize("zetas", [(1, 2, 4), (1, 4), (1, 16), (2, 8)])
+@pytest.mark.parametrize("cutoff", CUTOFFS)
+def test_powers_of_two_by_cutoff(gpu, monkeypatch, tmp_path, cutoff, zetas, n):
+    d = _pow2_potential(tmp_path / "p", cutoff, zetas)
+    pos, elem = _cluster(n, 2, n, 3.0)
+    _compare(d, pos, elem, None, monkeypatch)
+
+
 @pytest.mark.parametrize("zetas", [(1, 2, 4), (1, 2, 4, 16)])
 @pytest.mark.parametrize("cutoff", CUTOFFS + ["1 0.0"])
 def test_powers_of_two_by_cutoff_mixed(gpu, monkeypatch, tmp_path, cutoff,
@@ -116,3 +125,20 @@ def test_powers_of_two_by_cutoff_mixed(gpu, monkeypatch, tmp_path, cutoff,
         e, s = _rms([x - x0]), _rms([y - x0])
         print(f"{cutoff} {zetas}: {name} {e:.3e} / {s:.3e}")
         assert 0.0 < e <= 1.25 * s
+
+
+@pytest.mark.parametrize("pot", ["potentials/h2o_wtd", "potentials/h2o_52"])
+def test_storing_kernels_with_global_tables(gpu, monkeypatch, pot):
+    """Group tables in global memory are read by the kernels that form dG/dr,
+    which an evaluation on the two-pass path does not launch."""
+    d = os.path.join(GOLD, pot)
+    box, pos, elem = synth.water_box(64, 17)
+    out = []
+    for tables in (False, True):
+        if tables:
+            monkeypatch.setenv("N2P2B_SF_GLOBAL_TABLES", "1")
+        p = _prediction(d, True, monkeypatch)
+        e, f = p.predict(pos, elem, box)
+        out.append((np.array([e]), f, p.symmetry_functions(), p.dGdr()[0]))
+    for a, b in zip(*out):
+        assert np.abs(a - b).max() <= 1e-12 * np.abs(a).max()
