@@ -1405,15 +1405,20 @@ struct n2p2b_context
         launchNeighborList(L, stream);
     }
 
-    PairLaunch pairLaunch()
+    int multiprocessors()
     {
         if (smCount == 0)
             ck(cudaDeviceGetAttribute(&smCount, cudaDevAttrMultiProcessorCount,
                                       device), "device attribute");
+        return smCount;
+    }
+
+    PairLaunch pairLaunch()
+    {
         PairLaunch L;
         L.n = (int)n;
         L.cap = sfCap;
-        L.sms = smCount;
+        L.sms = multiprocessors();
         L.precision = precision;
         L.maxSF = maxSF;
         L.elem = elem.as<int>();
@@ -1789,6 +1794,7 @@ struct n2p2b_context
         L.elem = elem.as<int>();
         L.atomsByElem = atomsByElem.as<int>();
         L.es = es;
+        L.sms = multiprocessors();
         L.weights = stu.w.p;
         L.G = G.p;
         L.energy = Ei.as<double>();
@@ -2107,6 +2113,7 @@ struct n2p2b_context
         L.elem = elem.as<int>();
         L.atomsByElem = atomsByElem.as<int>();
         L.es = es;
+        L.sms = multiprocessors();
         L.weights = nnW.as<double>();
         L.G = G.as<double>();
         L.energy = Ei.as<double>();

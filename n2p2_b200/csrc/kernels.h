@@ -214,9 +214,11 @@ struct NNLaunch
     int           derivatives = 1;
     int           maxSF = 0;
     int           precision = PREC_FP64;  // type of weights, G and dE/dG
-    // Atoms by element (tiles of several atoms; null: per atom only).
+    // Atoms by element (tiles of several atoms; null: per atom only) and the
+    // device's multiprocessors, by which the launcher chooses tiles.
     int const*    atomsByElem = nullptr;
     ElemStarts    es{};
+    int           sms = 1;
     int const*    elem = nullptr;
     void const*   weights = nullptr;  // blob, offsets in NNParams
     void const*   G = nullptr;

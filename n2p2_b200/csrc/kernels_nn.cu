@@ -702,7 +702,7 @@ void launchNeuralNetworks(NNParams const& P, NNLaunch const& L,
 {
     // Tiles once every multiprocessor has four blocks of them, and where
     // their values fit.
-    if (L.atomsByElem && L.n >= kNNTile * kNNWarps * 4 * 148)
+    if (L.atomsByElem && L.n >= kNNTile * kNNWarps * 4 * L.sms)
     {
         NNTileLaunch N;
         N.L = L;
