@@ -230,14 +230,24 @@ def potential_shape(p):
     return M_a, M_r, S, n_sf
 
 
+# FP64 instructions that the two-pass kernels need for a valid triplet of the
+# timed potential (units of three runs, zeta 1, 2 and 4, cosine cutoff),
+# counted in their source: 77 for the values, 134 for each of the two owners
+# in the forces pass.  Staging, lane sums, idle lanes and pairs beyond the
+# cutoff are not counted.  A radial member's exponential, cutoff and
+# derivative take about 15.
+PAIR_OPS = (77, 2 * 134)
+RADIAL_OPS = 15
+
+
 def work_model(cnt, dr, d, shape, mac, rc=12.0):
     """Exact neighbor (n) and valid-triplet (T) counts of one frame and the
-    FLOP / byte model: per triplet 40 + 60 M_a, per (pair, radial member)
-    20, NN 3*2*MAC, chain rule 6 per Vec3D slot.  The FLOPs are those of the
-    plain formulation (dG/dr of every member, then the chain rule); the
-    kernels contract dE/dG inside the triplets and execute fewer.  Bytes of
-    the two symmetry-function kernels = neighbor data read twice, G written,
-    dE/dG read, pair and self terms written."""
+    FLOP / byte model of the two symmetry-function kernels: PAIR_OPS FP64
+    instructions per triplet, RADIAL_OPS per (pair, radial member) and pass
+    (an instruction counts as the two FLOPs of a fused multiply-add, as in
+    the DGEMM peak), NN 3*2*MAC, pair and self forces 6 per entry.  Bytes =
+    neighbor data read twice, G written, dE/dG read, pair and self terms
+    written."""
     import torch
     M_a, M_r, S, n_sf = shape
     dev = torch.device("cuda")
@@ -262,8 +272,8 @@ def work_model(cnt, dr, d, shape, mac, rc=12.0):
         m = (dd < rc2) & ok[:, :, None] & ok[:, None, :] & tri
         T += int(m.sum())
     n = int(cnt.sum())
-    flops_sf = T * (40 + 60 * M_a) + n * M_r * 20
-    flops_all = flops_sf + N * 3 * 2 * mac + 6 * (n * S + N * n_sf)
+    flops_sf = 2 * (T * sum(PAIR_OPS) + 2 * n * M_r * RADIAL_OPS)
+    flops_all = flops_sf + N * 3 * 2 * mac + 6 * n
     bytes_sf = n * (2 * 32 + 24) + N * n_sf * 8 * 2 + N * 24
     return {"atoms": N, "neighbors": n, "triplets": T,
             "neighbors_per_atom": n / N, "triplets_per_atom": T / N,
@@ -874,11 +884,10 @@ def run_ours(a):
             "peak_source": "cuBLAS DGEMM 8192^3 timed in this run "
                            "(builder-measured: the driver's peaks file has "
                            "no FP64 figure)",
-            "achieved_source": "counting-model FLOPs of the frame (exact "
-                               "triplet and neighbor counts, see work) / "
-                               "the CUDA-event time of the SF and force "
-                               "stages; the kernels execute fewer "
-                               "(dE/dG is contracted in the triplets)",
+            "achieved_source": "FP64 instructions that the kernels need for "
+                               "the frame's triplets and neighbors (exact "
+                               "counts, see work), two FLOPs each / the "
+                               "CUDA-event time of the SF and force stages",
             "algorithmic_flops_per_launch": wm["flops_sf"],
             "traffic": SF_TRAFFIC[0],
             "traffic_source": SF_TRAFFIC[1],
@@ -910,9 +919,10 @@ def profile_case(a):
     device times of the last three.  The symmetry-function kernel of
     evaluation k is that kernel's launch k (the first evaluation's sizing
     pass launches the neighbor list only).  --autotune runs the library's
-    tuner first and prints its choice; a capture that should see launch k
-    passes that choice through N2P2B_SF_VARIANT / N2P2B_SF_SORT instead,
-    because the tuner launches every configuration."""
+    tuner first and prints its choice; captures leave it out, because the
+    tuner launches every configuration.  N2P2B_SF_VARIANT / N2P2B_SF_SORT
+    ask for a variant of the storing kernels, and evaluations then run on
+    those instead of the two-pass ones."""
     from n2p2_b200 import synth
     from n2p2_b200.mode import Prediction
     box, pos, elem = synth.water_box(a.molecules, 77)
