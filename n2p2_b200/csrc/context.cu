@@ -869,7 +869,6 @@ struct n2p2b_context
         std::size_t const u = add(pt.units), r = add(pt.runs),
                           h = add(pt.shapes), q = add(pt.radials),
                           c = add(pt.cells), f = add(pt.fcs), w = add(pt.rads);
-        pt.p.units = pt.units.data();
         pairTabs.ensure(std::max<std::size_t>(blob.size(), 16));
         if (!blob.empty())
             ck(cudaMemcpy(pairTabs.p, blob.data(), blob.size(),

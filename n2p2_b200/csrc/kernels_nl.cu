@@ -15,7 +15,7 @@
 // own (j ascending; bc0, bc1, bc2 ascending) order.  Element grouping gives the
 // symmetry-function kernel contiguous per-element neighbor ranges.
 //
-// Two enumeration paths produce the same set:
+// Three enumeration paths produce the same set:
 //  * cell path: cells at least rc wide along every box vector, 27-cell stencil
 //    with periodic wrap.  Used when every box vector's perpendicular width
 //    exceeds rc (then pbc = 1) and every atom lies inside the cell (fractional
@@ -23,8 +23,11 @@
 //    |bc| <= 1 and sit in adjacent cells.  An FP32 distance decides away from
 //    the cutoff.  Hits are ranked by key per atom.
 //  * brute path: all (j, bc) candidates in key order, the reference's own
-//    enumeration; used for small or skewed cells, atoms outside the cell and
-//    non-periodic structures.
+//    enumeration; used for atoms outside the cell, open structures above the
+//    lane path's size and boxes with more than 128 images.
+//  * lane path (nlbLaneKernel): batches, structures of up to 640 atoms and
+//    boxes that cannot be cut into cells, with up to 128 images; only the
+//    images in reach are walked.
 #include "device_common.cuh"
 #include "kernels.h"
 
@@ -1026,18 +1029,8 @@ nlbLaneKernel(int n, int numElements, int NIMG,
                         imgDecode(p, img, b0, b1, b2);
                         double dr[3];
                         nlTest(p, ri, pos, j, b0, b1, b2, dr);
-                        double const n2 = __dadd_rn(
-                            __dadd_rn(__dmul_rn(dr[0], dr[0]),
-                                      __dmul_rn(dr[1], dr[1])),
-                            __dmul_rn(dr[2], dr[2]));
-                        out.key[o] = nlKey(e, j, img, n, NIMG);
-                        out.nbrIdx[o] = j;
-                        out.nbrEl[o] = (int8_t)e;
-                        out.dx[o] = dr[0];
-                        out.dy[o] = dr[1];
-                        out.dz[o] = dr[2];
-                        out.dd[o] = __dsqrt_rn(n2);
-                        out.entryAtom[o] = i;
+                        writeEntry(out, o, i, nlKey(e, j, img, n, NIMG), j,
+                                   e, dr);
                         ++o;
                     }
                 }
