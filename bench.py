@@ -536,9 +536,10 @@ def measure_forms(box, frames, elem, dev_frames, stream, lib, steps, local):
                                          "bohr")
     out["forms"] = {
         "fp64": "plain form, everything FP64",
-        "mixed": "FP32 symmetry functions + dG/dr; NN on tcgen05 with BF16 "
-                 "hi/lo operand pairs (3 MMAs per step), FP32 accumulation; "
-                 "FP64 displacements, energy sum, force accumulation",
+        "mixed": "FP32 symmetry functions and force terms; NN on tcgen05 "
+                 "with BF16 hi/lo operand pairs (3 MMAs per step), FP32 "
+                 "accumulation; FP64 displacements, energy sum, sums of the "
+                 "force terms",
         "bf16": "as mixed, except single BF16 deltas against hi/lo "
                 "weights in the backward GEMMs of the hidden layers above "
                 "the first (2 MMAs per step there); meets_targets says "

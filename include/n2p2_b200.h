@@ -66,10 +66,10 @@ int         n2p2b_set_stream(n2p2b_context* ctx, void* stream);
 
 /* Arithmetic of the evaluation.  No counterpart in the reference (it always
  * computes in double).  N2P2B_PRECISION_FP64 (default) is the plain form.
- * The two mixed forms compute symmetry functions and dG/dr in FP32 and the
- * atomic NNs on the tensor cores with BF16 operands and FP32 accumulation;
- * neighbor displacements, the energy sum and the force accumulation stay
- * FP64.  N2P2B_PRECISION_MIXED splits each NN operand into BF16 high and low
+ * The two mixed forms compute symmetry functions, dG/dr and the force terms
+ * of single triplets in FP32 and the atomic NNs on the tensor cores with BF16
+ * operands and FP32 accumulation; neighbor displacements, the energy sum and
+ * the sums of the force terms stay FP64.  N2P2B_PRECISION_MIXED splits each NN operand into BF16 high and low
  * parts (three tensor-core products per step, about 16 significant bits);
  * N2P2B_PRECISION_BF16 splits the operands of the forward sweep and of
  * dE/dG as MIXED does and keeps the back-propagated derivatives of the

@@ -186,7 +186,7 @@ void launchPair(int pass, SFParams const& P, PairParams const& host,
     //          0.154 / 0.168, 24,576 0.97 / 1.16);
     //  forces  enough waves to even out the atoms' unequal work (FP64: 6,000
     //          atoms 0.68 / 0.64, 9,000 0.92 / 0.94, 24,576 2.41 / 2.52; FP32,
-    //          92 functions: 4,200 0.357 / 0.351, 6,000 0.477 / 0.488);
+    //          92 functions: 4,200 0.370 / 0.365, 6,000 0.495 / 0.510);
     //          atoms of few neighbors have too few items of eight owners for
     //          four warps (1,728 atoms of Cu2S 0.267 / 0.308).
     L.wpa = 1;

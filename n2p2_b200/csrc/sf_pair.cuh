@@ -45,7 +45,7 @@
 // per owner for the forces, 3 runs x 4 shapes) and their latency at 12 to 16
 // warps per multiprocessor bound both passes.  24,576 water atoms, 52
 // functions, FP64: 0.96 + 2.4 ms, where dG/dr took 6.1 to form and 0.4 to
-// contract (2 GB each way); 98,304 atoms, 92 functions, FP32: 2.7 + 6.8 ms
+// contract (2 GB each way); 98,304 atoms, 92 functions, FP32: 2.8 + 7.0 ms
 // against 25.1 + 1.5.
 #pragma once
 
