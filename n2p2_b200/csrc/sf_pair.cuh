@@ -979,7 +979,7 @@ __device__ __forceinline__ void pow2Values(SFParams const& P,
         }
     });
     // Slots the unit does not have hold zeros and have no cells.
-    flushCells<R, NZ * NR * 2>(w, acc, u.cell, pairUnitCells(u));
+    flushCells<R, NZ * NR * 2>(w, acc, u.cell, pairUnitCells<PK_POW2>(u));
 }
 
 template <typename R, int CT, int NR, bool NARROW>
@@ -1102,7 +1102,8 @@ __device__ __forceinline__ void generalValues(SFParams const& P,
                 for (int q = 0; q < S; ++q) acc[a * S + q] += v * phi[q];
             }
     });
-    flushCells<R, kPairGenRuns * S>(w, acc, u.cell, pairUnitCells(u));
+    flushCells<R, kPairGenRuns * S>(w, acc, u.cell,
+                                    pairUnitCells<PK_GENERAL>(u));
 }
 
 template <typename R, bool NARROW>
@@ -1152,7 +1153,7 @@ __device__ __forceinline__ void compactValues(SFParams const& P,
                 for (int s = 0; s < S; ++s) acc[a * S + s] += v * phi[s];
             }
     });
-    flushCells<R, N>(w, acc, u.cell, pairUnitCells(u));
+    flushCells<R, N>(w, acc, u.cell, pairUnitCells<PK_COMPACT>(u));
 }
 
 template <typename R, int CT, int NZ, int MASK, bool NARROW>

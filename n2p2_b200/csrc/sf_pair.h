@@ -66,20 +66,18 @@ struct PairUnit
     double   zeta[4];     // ladder
 };
 
-// Cells of a unit.  PK_POW2 units have those of PairParams::slots values of
+// Cells of a unit of kind KIND.  PK_POW2 units have those of PairParams::slots values of
 // zeta, which may be fewer than the slots a kernel is compiled for: kernels
 // touch these cells and no others.
+template <int KIND>
 #ifdef __CUDACC__
 __host__ __device__
 #endif
 inline int pairUnitCells(PairUnit const& u)
 {
-    switch (u.kind)
-    {
-    case PK_GENERAL: return u.nr * kPairGenShapes;
-    case PK_COMPACT: return u.nr * kPairCompShapes;
-    default: return 2 * u.nr * u.ns;
-    }
+    if (KIND == PK_GENERAL) return u.nr * kPairGenShapes;
+    if (KIND == PK_COMPACT) return u.nr * kPairCompShapes;
+    return 2 * u.nr * u.ns;
 }
 
 struct PairRun

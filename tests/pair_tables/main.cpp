@@ -13,6 +13,17 @@
 
 using namespace n2p2b;
 
+static int cells(PairUnit const& u)
+{
+    switch (u.kind)
+    {
+    case PK_POW2: return pairUnitCells<PK_POW2>(u);
+    case PK_LADDER: return pairUnitCells<PK_LADDER>(u);
+    case PK_GENERAL: return pairUnitCells<PK_GENERAL>(u);
+    default: return pairUnitCells<PK_COMPACT>(u);
+    }
+}
+
 int main()
 {
     SFParams P{};
@@ -62,8 +73,7 @@ int main()
     {
         for (int u = t.p.unitBeg[k]; u < t.p.unitBeg[k + 1]; ++u)
             std::cout << "unit " << k << " " << t.units[u].kind << " "
-                      << t.units[u].cell << " " << pairUnitCells(t.units[u])
-                      << "\n";
+                      << t.units[u].cell << " " << cells(t.units[u]) << "\n";
         for (int r = t.p.radialBeg[k]; r < t.p.radialBeg[k + 1]; ++r)
             std::cout << "radial " << k << " " << t.radials[r].cell << "\n";
         std::cout << "cells " << k << " "
